@@ -5,26 +5,34 @@
 // :527 batched 3-centre, :595 2-centre).
 //
 // Work is bucketed by angular-momentum class so every warp runs one class:
-// one launch per (la,lb[,lc]) class, one thread per shell pair (1e, Schwarz),
-// per (shell pair, aux shell) triplet (3-centre) or per aux pair (2-centre).
+// one launch per (la,lb[,lc]) class, a group of lanes per shell pair (1e,
+// Schwarz) or (shell pair, aux shell) triplet (3-centre), which share its
+// primitive pairs, and one thread per aux pair (2-centre). The recursions are
+// unrolled with constant indices (ints_unrolled.cuh).
 //
 // Conventions: Cartesian components in lexicographic order (xx,xy,xz,yy,yz,zz);
-// contracted shells normalised so the x^l component has unit norm; the
-// "unit shell" (exponent 0, coefficient 1) turns 4-centre into 3-/2-centre
-// integrals, as in libCMS/CMS_Simint.c:131-141.
+// contracted shells normalised so the x^l component has unit norm; a second
+// exponent of 0 turns 4-centre into 3-/2-centre integrals, as the unit shell
+// of libCMS/CMS_Simint.c:131-141 does.
 #include <cmath>
 #include <cstdio>
+#include <map>
+#include <mutex>
 #include <vector>
 
+#include "ints_unrolled.cuh"
 #include "tscf_internal.h"
 #include "tune.h"
 
 namespace tscf {
 
+using namespace unrolled;
+
 // ------------------------------------------------------------------ tables
 // Cartesian components of every level l <= 8 in cumulative order:
-// index ncum(l-1) + n(n+1)/2 + lz with n = l - lx.
+// index ncum(l-1) + n(n+1)/2 + lz with n = l - lx (read by the run-time recursion).
 __constant__ unsigned char c_comp[165][3];
+// F_m at the grid points T = k BOYS_DT, m = 0 .. 15
 __device__ double g_boys[BOYS_NGRID * 16];
 
 static bool g_tables_ready[64] = {false};
@@ -68,6 +76,157 @@ void boys_table_init(cudaStream_t s)
     cudaMemcpyToSymbolAsync(c_comp, comp, sizeof(comp), 0, cudaMemcpyHostToDevice, s);
     cudaStreamSynchronize(s);
     if (dev < 64) g_tables_ready[dev] = true;
+}
+
+struct Sh {
+    int am, np;
+    double x, y, z;
+    const double *al, *co;
+};
+__device__ __forceinline__ Sh load_shell(const DevShells &s, int i)
+{
+    Sh r;
+    r.am = s.am[i];
+    r.np = s.nprim[i];
+    r.x = s.cen[3 * i];
+    r.y = s.cen[3 * i + 1];
+    r.z = s.cen[3 * i + 2];
+    r.al = s.alpha + s.poff[i];
+    r.co = s.coef + s.poff[i];
+    return r;
+}
+
+// ------------------------------------------------------------------ class launches side by side
+// The angular-momentum classes of one integral kind write disjoint outputs, and
+// a small molecule's classes are a few blocks each whose threads run their
+// primitives as a serial chain (0.1 to 1.4 ms per class on water): one after
+// another on one stream they leave the chip idle. A Fork runs them on LANES
+// streams between an event on the caller's stream and events that it waits for.
+// Streams and events come from a per-device pool of at most KEEP sets (a set
+// belongs to one Fork at a time), so nothing is created per call.
+class Fork {
+    static constexpr int LANES = 8, KEEP = 4;
+    struct Set {
+        cudaStream_t st[LANES] = {};
+        cudaEvent_t begin = nullptr, done[LANES] = {};
+        bool ok = true;
+        Set()
+        {
+            ok = cudaEventCreateWithFlags(&begin, cudaEventDisableTiming) == cudaSuccess;
+            for (int k = 0; k < LANES; k++)
+                ok = ok && cudaStreamCreateWithFlags(&st[k], cudaStreamNonBlocking) == cudaSuccess &&
+                     cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming) == cudaSuccess;
+        }
+        ~Set()
+        {
+            for (int k = 0; k < LANES; k++) {
+                if (st[k]) cudaStreamDestroy(st[k]);
+                if (done[k]) cudaEventDestroy(done[k]);
+            }
+            if (begin) cudaEventDestroy(begin);
+        }
+    };
+    static std::mutex &lock()
+    {
+        static std::mutex *m = new std::mutex;
+        return *m;
+    }
+    static std::vector<Set *> &pool(int dev)
+    {
+        static auto *p = new std::map<int, std::vector<Set *>>;   // outlives static destruction
+        return (*p)[dev];
+    }
+    int dev_ = 0, n_ = 0;
+    cudaStream_t s_;
+    Set *set_ = nullptr;
+
+public:
+    // side = false: every launch stays on s
+    Fork(cudaStream_t s, bool side) : s_(s)
+    {
+        if (!side) return;
+        cudaGetDevice(&dev_);
+        {
+            std::lock_guard<std::mutex> g(lock());
+            auto &v = pool(dev_);
+            if (!v.empty()) {
+                set_ = v.back();
+                v.pop_back();
+            }
+        }
+        if (!set_) set_ = new Set;
+        if (!set_->ok || cudaEventRecord(set_->begin, s) != cudaSuccess) {
+            cudaGetLastError();
+            delete set_;
+            set_ = nullptr;
+        }
+    }
+    Fork(const Fork &) = delete;
+    Fork &operator=(const Fork &) = delete;
+    cudaStream_t next()
+    {
+        if (!set_) return s_;
+        const int k = n_++ % LANES;
+        if (n_ <= LANES) cudaStreamWaitEvent(set_->st[k], set_->begin, 0);
+        return set_->st[k];
+    }
+    ~Fork()
+    {
+        if (!set_) return;
+        for (int k = 0; k < LANES && k < n_; k++) {
+            cudaEventRecord(set_->done[k], set_->st[k]);
+            cudaStreamWaitEvent(s_, set_->done[k], 0);
+        }
+        std::lock_guard<std::mutex> g(lock());
+        auto &v = pool(dev_);
+        if ((int) v.size() < KEEP) v.push_back(set_);
+        else delete set_;
+    }
+};
+
+// ------------------------------------------------------------------ primitive quartets, unrolled
+constexpr double TWO_PI_52 = 2.0 * 17.493418327624862;   // 2 pi^2.5
+constexpr int INT_THREADS = 128;                         // most threads per block of the pair kernels
+
+// Primitive pair kp of shells A, B (kp = ka * B.np + kb; beyond the last one: a zero prefactor).
+__device__ __forceinline__ PrimPair prim_pair(const Sh &A, const Sh &B, double AB2, int kp)
+{
+    PrimPair t{1.0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (kp < A.np * B.np) {
+        const int ka = kp / B.np, kb = kp - ka * B.np;
+        const double a = A.al[ka], b = B.al[kb];
+        t.z = a + b;
+        t.iz = 1.0 / t.z;
+        t.x = (a * A.x + b * B.x) * t.iz;
+        t.y = (a * A.y + b * B.y) * t.iz;
+        t.zc = (a * A.z + b * B.z) * t.iz;
+        t.k = A.co[ka] * B.co[kb] * exp(-a * b * t.iz * AB2);
+        t.b = b;
+    }
+    return t;
+}
+
+// Adds scale * [e|f], e = ELO..EHI, f = FLO..FHI, of one primitive quartet to acc. P: the bra pair with A's
+// centre (ax, ay, az); q: the ket pair (eta, 1/eta, centre, prefactor, its second exponent d).
+template <int ELO, int EHI, int FLO, int FHI>
+__device__ __forceinline__ void quartet_add(const PrimPair &p, const double (&A)[3], const double (&AB)[3],
+                                            const PrimPair &q, const double (&CD)[3], double scale,
+                                            double (&acc)[(ncum(EHI) - ncum(ELO - 1)) * (ncum(FHI) - ncum(FLO - 1))])
+{
+    constexpr int L = EHI + FHI;
+    const double izt = 1.0 / (p.z + q.z), rho = p.z * q.z * izt;
+    const double QP[3] = {q.x - p.x, q.y - p.y, q.zc - p.zc};
+    const double T = rho * (QP[0] * QP[0] + QP[1] * QP[1] + QP[2] * QP[2]);
+    const double pref = TWO_PI_52 * p.iz * q.iz * sqrt(izt) * p.k * q.k;
+    double F[L + 1], e0[ncum(L)];
+    boys_scaled<L>(g_boys, T, pref, F);
+    const double PA[3] = {p.x - A[0], p.y - A[1], p.zc - A[2]};
+    const double w = q.z * izt;   // W - P = eta / (zeta + eta) (Q - P)
+    const double WP[3] = {w * QP[0], w * QP[1], w * QP[2]};
+    vrr<L>(F, PA, WP, 0.5 * p.iz, rho * p.iz, e0);
+    const double cAB[3] = {-(p.b * AB[0] + q.b * CD[0]) * q.iz, -(p.b * AB[1] + q.b * CD[1]) * q.iz,
+                           -(p.b * AB[2] + q.b * CD[2]) * q.iz};
+    etr_add<ELO, EHI, FLO, FHI>(e0, cAB, 0.5 * q.iz, p.z * q.iz, scale, acc);
 }
 
 // F_m(T), m = 0..mmax: 7-term Taylor expansion of F_mmax about the nearest grid
@@ -236,56 +395,6 @@ __device__ __forceinline__ void etr_accumulate(int L, int la, int Le, int lc, in
     }
 }
 
-// HRR leaves of (a,b| for lb <= 2: (a,b| = sum_k w_k (e_k,0| with AB = A - B.
-__device__ __forceinline__ int hrr_leaves(int ax, int ay, int az, int bx, int by, int bz, const double AB[3],
-                                          int *e, double *w)
-{
-    int lb = bx + by + bz;
-    if (lb == 0) {
-        e[0] = cum_of(ax, ay, az);
-        w[0] = 1.0;
-        return 1;
-    }
-    int i = bx > 0 ? 0 : (by > 0 ? 1 : 2);
-    int di[3] = {i == 0, i == 1, i == 2};
-    if (lb == 1) {
-        e[0] = cum_of(ax + di[0], ay + di[1], az + di[2]);
-        w[0] = 1.0;
-        e[1] = cum_of(ax, ay, az);
-        w[1] = AB[i];
-        return 2;
-    }
-    int rx = bx - di[0], ry = by - di[1];
-    int j = rx > 0 ? 0 : (ry > 0 ? 1 : 2);
-    int dj[3] = {j == 0, j == 1, j == 2};
-    e[0] = cum_of(ax + di[0] + dj[0], ay + di[1] + dj[1], az + di[2] + dj[2]);
-    w[0] = 1.0;
-    e[1] = cum_of(ax + di[0], ay + di[1], az + di[2]);
-    w[1] = AB[j];
-    e[2] = cum_of(ax + dj[0], ay + dj[1], az + dj[2]);
-    w[2] = AB[i];
-    e[3] = cum_of(ax, ay, az);
-    w[3] = AB[i] * AB[j];
-    return 4;
-}
-
-struct Sh {
-    int am, np;
-    double x, y, z;
-    const double *al, *co;
-};
-__device__ __forceinline__ Sh load_shell(const DevShells &s, int i)
-{
-    Sh r;
-    r.am = s.am[i];
-    r.np = s.nprim[i];
-    r.x = s.cen[3 * i];
-    r.y = s.cen[3 * i + 1];
-    r.z = s.cen[3 * i + 2];
-    r.al = s.alpha + s.poff[i];
-    r.co = s.coef + s.poff[i];
-    return r;
-}
 __device__ __forceinline__ Sh unit_shell()
 {
     Sh r;
@@ -347,6 +456,39 @@ __device__ void quartet_acc(const Sh &A, const Sh &B, bool ub, const Sh &C, cons
     }
 }
 
+// HRR leaves of (a,b| for lb <= 2: (a,b| = sum_k w_k (e_k,0| with AB = A - B.
+__device__ __forceinline__ int hrr_leaves(int ax, int ay, int az, int bx, int by, int bz, const double AB[3],
+                                          int *e, double *w)
+{
+    int lb = bx + by + bz;
+    if (lb == 0) {
+        e[0] = cum_of(ax, ay, az);
+        w[0] = 1.0;
+        return 1;
+    }
+    int i = bx > 0 ? 0 : (by > 0 ? 1 : 2);
+    int di[3] = {i == 0, i == 1, i == 2};
+    if (lb == 1) {
+        e[0] = cum_of(ax + di[0], ay + di[1], az + di[2]);
+        w[0] = 1.0;
+        e[1] = cum_of(ax, ay, az);
+        w[1] = AB[i];
+        return 2;
+    }
+    int rx = bx - di[0], ry = by - di[1];
+    int j = rx > 0 ? 0 : (ry > 0 ? 1 : 2);
+    int dj[3] = {j == 0, j == 1, j == 2};
+    e[0] = cum_of(ax + di[0] + dj[0], ay + di[1] + dj[1], az + di[2] + dj[2]);
+    w[0] = 1.0;
+    e[1] = cum_of(ax + di[0], ay + di[1], az + di[2]);
+    w[1] = AB[j];
+    e[2] = cum_of(ax + dj[0], ay + dj[1], az + dj[2]);
+    w[2] = AB[i];
+    e[3] = cum_of(ax, ay, az);
+    w[3] = AB[i] * AB[j];
+    return 4;
+}
+
 // ------------------------------------------------------------------ 3-centre kernel
 // One thread per (shell pair in class, aux shell of AM lc). Writes pqA_u rows.
 // aux_major = 0: consecutive threads take consecutive aux shells of one pair;
@@ -399,6 +541,13 @@ __global__ void __launch_bounds__(256) k_three_center(DevShells sh, DevShells au
     }
 }
 
+static std::string key_3c(int la, int lb, int lc, long long n)
+{
+    char key[64];
+    snprintf(key, sizeof(key), "3c:%d%d%d:%s", la, lb, lc, n < 65536 ? "small" : "large");
+    return key;
+}
+
 template <int LA, int LB, int LC>
 static void launch_3c_class(const DevShells &sh, const DevShells &aux, const ThreeCenterPlan &pl, int pair0,
                             int npairs, int lc_start, int naux_am, double *pqA, cudaStream_t s)
@@ -414,8 +563,7 @@ static void launch_3c_class(const DevShells &sh, const DevShells &aux, const Thr
         g_launches++;
     };
     // every candidate writes the same values, so re-running while tuning is harmless
-    char key[64];
-    snprintf(key, sizeof(key), "3c:%d%d%d:%s", LA, LB, LC, n < 65536 ? "small" : "large");
+    const std::string key = key_3c(LA, LB, LC, n);
     int c = tune_lookup(key);
     if (c < 0 && tune_enabled()) {
         tune_run(key, {0, 1, 2, 3, 4, 5}, run, s, 1);
@@ -426,40 +574,61 @@ static void launch_3c_class(const DevShells &sh, const DevShells &aux, const Thr
 
 template <int LA, int LB>
 static void launch_3c_lc(const DevShells &sh, const DevShells &aux, const ThreeCenterPlan &pl, int pair0, int np,
-                         double *pqA, cudaStream_t s)
+                         double *pqA, Fork &f)
 {
     for (int lc = 0; lc <= MAX_L_AUX; lc++) {
         int st = pl.aux_am_start[lc], cnt = pl.aux_am_start[lc + 1] - st;
+        if (cnt == 0) continue;
         switch (lc) {
-        case 0: launch_3c_class<LA, LB, 0>(sh, aux, pl, pair0, np, st, cnt, pqA, s); break;
-        case 1: launch_3c_class<LA, LB, 1>(sh, aux, pl, pair0, np, st, cnt, pqA, s); break;
-        case 2: launch_3c_class<LA, LB, 2>(sh, aux, pl, pair0, np, st, cnt, pqA, s); break;
-        case 3: launch_3c_class<LA, LB, 3>(sh, aux, pl, pair0, np, st, cnt, pqA, s); break;
+        case 0: launch_3c_class<LA, LB, 0>(sh, aux, pl, pair0, np, st, cnt, pqA, f.next()); break;
+        case 1: launch_3c_class<LA, LB, 1>(sh, aux, pl, pair0, np, st, cnt, pqA, f.next()); break;
+        case 2: launch_3c_class<LA, LB, 2>(sh, aux, pl, pair0, np, st, cnt, pqA, f.next()); break;
+        case 3: launch_3c_class<LA, LB, 3>(sh, aux, pl, pair0, np, st, cnt, pqA, f.next()); break;
         }
     }
+}
+
+// Whether a class of the plan still has its block shape to be timed (alone on its stream).
+static bool tuning_3c(const ThreeCenterPlan &pl)
+{
+    if (!tune_enabled()) return false;
+    for (int c = 0; c < pl.nclass; c++)
+        for (int lc = 0; lc <= MAX_L_AUX; lc++) {
+            const long long n = (long long) (pl.class_start[c + 1] - pl.class_start[c]) *
+                                (pl.aux_am_start[lc + 1] - pl.aux_am_start[lc]);
+            if (n > 0 && tune_lookup(key_3c(pl.class_la[c], pl.class_lb[c], lc, n)) < 0) return true;
+        }
+    return false;
 }
 
 void launch_three_center(const DevShells &sh, const DevShells &aux, const ThreeCenterPlan &pl, double *pqA,
                          cudaStream_t s)
 {
+    Fork f(s, !tuning_3c(pl));
     for (int c = 0; c < pl.nclass; c++) {
         int p0 = pl.class_start[c], np = pl.class_start[c + 1] - p0;
         if (np == 0) continue;
         int la = pl.class_la[c], lb = pl.class_lb[c];
         int key = la * 3 + lb;
         switch (key) {
-        case 0: launch_3c_lc<0, 0>(sh, aux, pl, p0, np, pqA, s); break;
-        case 3: launch_3c_lc<1, 0>(sh, aux, pl, p0, np, pqA, s); break;
-        case 4: launch_3c_lc<1, 1>(sh, aux, pl, p0, np, pqA, s); break;
-        case 6: launch_3c_lc<2, 0>(sh, aux, pl, p0, np, pqA, s); break;
-        case 7: launch_3c_lc<2, 1>(sh, aux, pl, p0, np, pqA, s); break;
-        case 8: launch_3c_lc<2, 2>(sh, aux, pl, p0, np, pqA, s); break;
+        case 0: launch_3c_lc<0, 0>(sh, aux, pl, p0, np, pqA, f); break;
+        case 3: launch_3c_lc<1, 0>(sh, aux, pl, p0, np, pqA, f); break;
+        case 4: launch_3c_lc<1, 1>(sh, aux, pl, p0, np, pqA, f); break;
+        case 6: launch_3c_lc<2, 0>(sh, aux, pl, p0, np, pqA, f); break;
+        case 7: launch_3c_lc<2, 1>(sh, aux, pl, p0, np, pqA, f); break;
+        case 8: launch_3c_lc<2, 2>(sh, aux, pl, p0, np, pqA, f); break;
         default: break;   // la < lb never occurs: pairs are oriented with am(M) >= am(N)
         }
     }
 }
 
 // ------------------------------------------------------------------ 2-centre kernel
+// The (P|Q) kernel keeps the recursion with run-time loops, bit for bit: with
+// the metric's condition number (6e10 on C40H82) another rounding of (P|Q)
+// re-rolls the rounding of its explicit inverse square root, which shifts a
+// molecule's energy by up to 1e-8 Eh (measured on C40H82: 1.3e-8 between this
+// kernel and one on the unrolled recursion). It takes 1.3 ms of a C40H82's
+// set-up; the unrolled one took 0.26 ms.
 template <int LP, int LQ>
 __global__ void __launch_bounds__(128) k_two_center(DevShells aux, const int *idsP, int nP, const int *idsQ, int nQ,
                                                     const double *df_scr, double scrtol2, double *Jpq, int naux)
@@ -490,7 +659,7 @@ struct AuxGroups {
 
 template <int LP>
 static void launch_2c_row(const DevShells &aux, const AuxGroups &g, const double *df_scr, double scrtol2, double *Jpq,
-                          int naux, cudaStream_t s)
+                          int naux, Fork &f)
 {
     for (int lq = 0; lq <= MAX_L_AUX; lq++) {
         int p0 = g.start[LP], nP = g.start[LP + 1] - p0;
@@ -499,10 +668,10 @@ static void launch_2c_row(const DevShells &aux, const AuxGroups &g, const double
         if (n == 0) continue;
         int blocks = (int) ((n + 127) / 128);
         switch (lq) {
-        case 0: k_two_center<LP, 0><<<blocks, 128, 0, s>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
-        case 1: k_two_center<LP, 1><<<blocks, 128, 0, s>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
-        case 2: k_two_center<LP, 2><<<blocks, 128, 0, s>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
-        case 3: k_two_center<LP, 3><<<blocks, 128, 0, s>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
+        case 0: k_two_center<LP, 0><<<blocks, 128, 0, f.next()>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
+        case 1: k_two_center<LP, 1><<<blocks, 128, 0, f.next()>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
+        case 2: k_two_center<LP, 2><<<blocks, 128, 0, f.next()>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
+        case 3: k_two_center<LP, 3><<<blocks, 128, 0, f.next()>>>(aux, g.ids + p0, nP, g.ids + q0, nQ, df_scr, scrtol2, Jpq, naux); break;
         }
     }
 }
@@ -511,95 +680,172 @@ void launch_two_center_grouped(const DevShells &aux, const int *d_ids, const int
                                double scrtol2, double *d_Jpq, int naux, cudaStream_t s)
 {
     AuxGroups g{d_ids, h_start};
-    launch_2c_row<0>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, s);
-    launch_2c_row<1>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, s);
-    launch_2c_row<2>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, s);
-    launch_2c_row<3>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, s);
+    Fork f(s, true);
+    launch_2c_row<0>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, f);
+    launch_2c_row<1>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, f);
+    launch_2c_row<2>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, f);
+    launch_2c_row<3>(aux, g, d_df_scr, scrtol2, d_Jpq, naux, f);
 }
 
 // max_p (p|p) per aux shell (the DF screening value).
+template <int L>
+__device__ __forceinline__ double aux_self_max(const Sh &A)
+{
+    constexpr int n = ncart(L);
+    double acc[n * n];
+#pragma unroll
+    for (int k = 0; k < n * n; k++) acc[k] = 0.0;
+    const double Ac[3] = {A.x, A.y, A.z}, none[3] = {0.0, 0.0, 0.0};
+    for (int ka = 0; ka < A.np; ka++)
+        for (int kc = 0; kc < A.np; kc++) {
+            const PrimPair p{A.al[ka], 1.0 / A.al[ka], A.x, A.y, A.z, A.co[ka], 0.0};
+            const PrimPair q{A.al[kc], 1.0 / A.al[kc], A.x, A.y, A.z, A.co[kc], 0.0};
+            quartet_add<L, L, L, L>(p, Ac, none, q, none, 1.0, acc);
+        }
+    double mx = 0.0;
+#pragma unroll
+    for (int k = 0; k < n; k++) mx = fmax(mx, fabs(acc[k * n + k]));
+    return mx;
+}
+
 __global__ void k_df_scrval(DevShells aux, double *out)
 {
-    int P = blockIdx.x * blockDim.x + threadIdx.x;
+    const int P = blockIdx.x * blockDim.x + threadIdx.x;
     if (P >= aux.nsh) return;
-    const Sh A = load_shell(aux, P), U = unit_shell();
-    double acc[ncart(MAX_L_AUX) * ncart(MAX_L_AUX)];
-    const int n = ncart(A.am);
-    quartet_acc<2 * MAX_L_AUX, MAX_L_AUX>(A, U, true, A, U, true, acc, n, n);
-    double mx = 0.0;
-    for (int k = 0; k < n; k++) mx = fmax(mx, fabs(acc[k * n + k]));
-    out[P] = mx;
+    const Sh A = load_shell(aux, P);
+    switch (A.am) {
+    case 0: out[P] = aux_self_max<0>(A); break;
+    case 1: out[P] = aux_self_max<1>(A); break;
+    case 2: out[P] = aux_self_max<2>(A); break;
+    default: out[P] = aux_self_max<3>(A); break;
+    }
 }
 
 void launch_df_scrval(const DevShells &aux, double *d_out, cudaStream_t s)
 {
-    k_df_scrval<<<(aux.nsh + 63) / 64, 64, 0, s>>>(aux, d_out);
+    k_df_scrval<<<(aux.nsh + 31) / 32, 32, 0, s>>>(aux, d_out);
 }
 
 // ------------------------------------------------------------------ Schwarz kernel
-// (MN|MN): only the diagonal (mn|mn) elements are formed, each from its HRR
-// leaves on both sides. bf_scr[iM][iN] takes the element the reference reads
-// at iN*(dM*dN*dM+dM) + iM*(dN*dM+1) (TinySCF.c:153): the diagonal of the
-// component pair k = iN*dM + iM in the [dM][dN] ordering.
+// (MN|MN) for the unordered shell pairs of a class, LM >= LN: only the
+// diagonal (mn|mn) elements, each from its HRR leaves on both sides. SL lanes
+// share a pair's primitive quartets: lane sl takes the bra primitive pairs
+// p = sl, sl + SL, ..., the ket pairs q <= p come from a shared table that the
+// lanes fill SL at a time, and q < p counts twice ((p|q) = (q|p) on the
+// diagonal). bf_scr[iM][iN] takes the element the reference reads at
+// iN*(dM*dN*dM+dM) + iM*(dN*dM+1) (TinySCF.c:153): the diagonal of the
+// component pair k = iN*dM + iM in the [dM][dN] ordering; the swapped pair's
+// block is the same diagonal read with its own permutation.
+//
+// A pair of 8-primitive shells has 4096 primitive quartets; one thread per
+// ordered pair ran them as one serial chain (2 to 3 ms per class however few
+// pairs there were).
 template <int LM, int LN>
-__global__ void __launch_bounds__(64) k_schwarz(DevShells sh, const int *idsM, int nM, const int *idsN, int nN,
-                                                double *sp_scr, double *bf_scr, int nbf)
+__global__ void __launch_bounds__(INT_THREADS) k_schwarz(DevShells sh, const int *idsM, int nM, const int *idsN,
+                                                         int nN, double *sp_scr, double *bf_scr, int nbf, int SL)
 {
-    const long long tid = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= (long long) nM * nN) return;
-    const int M = idsM[tid / nN], N = idsN[tid % nN];
-    constexpr int dM = ncart(LM), dN = ncart(LN);
-    constexpr int NEa = ncum(LM + LN) - ncum(LM - 1);
-    double acc[NEa * NEa];
+    __shared__ PrimPair tab[INT_THREADS];
+    const int lane = threadIdx.x & 31, sl = lane & (SL - 1);
+    const long long npair = LM == LN ? (long long) nM * (nM + 1) / 2 : (long long) nM * nN;
+    const long long g = ((long long) blockIdx.x * blockDim.x + threadIdx.x) / SL;
+    const long long w0 = ((long long) blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / SL;
+    if (w0 >= npair) return;                       // the whole warp
+    const long long pr = g < npair ? g : npair - 1;
+    int iM, iN;
+    if (LM == LN) {                                // row iM of the lower triangle
+        iM = (int) ((sqrt(8.0 * (double) pr + 1.0) - 1.0) * 0.5);
+        while ((long long) iM * (iM + 1) / 2 > pr) iM--;
+        while ((long long) (iM + 1) * (iM + 2) / 2 <= pr) iM++;
+        iN = (int) (pr - (long long) iM * (iM + 1) / 2);
+    } else {
+        iM = (int) (pr / nN);
+        iN = (int) (pr % nN);
+    }
+    const int M = idsM[iM], N = idsN[iN];
+    constexpr int dM = ncart(LM), dN = ncart(LN), LE = LM + LN;
+    constexpr int NE = ncum(LE) - ncum(LM - 1), E0 = ncum(LM - 1);
+    double acc[NE * NE];
+#pragma unroll
+    for (int k = 0; k < NE * NE; k++) acc[k] = 0.0;
     const Sh A = load_shell(sh, M), B = load_shell(sh, N);
-    quartet_acc<(2 * (LM + LN) > 0 ? 2 * (LM + LN) : 1), LM + LN>(A, B, false, A, B, false, acc, NEa, NEa);
-    const double AB[3] = {A.x - B.x, A.y - B.y, A.z - B.z};
-    const int eoff = ncum(LM - 1);
-    const int baseA = ncum(LM - 1), baseB = ncum(LN - 1);
+    const double Ac[3] = {A.x, A.y, A.z}, AB[3] = {A.x - B.x, A.y - B.y, A.z - B.z};
+    const double AB2 = AB[0] * AB[0] + AB[1] * AB[1] + AB[2] * AB[2];
+    const int npp = A.np * B.np;
+    int most = npp;                                // over the warp: its pairs run the same chunks
+    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    PrimPair *t = tab + (threadIdx.x & ~(SL - 1));
+    for (int pb = 0; pb < most; pb += SL) {
+        const PrimPair p = prim_pair(A, B, AB2, pb + sl);
+        for (int qb = 0; qb <= pb; qb += SL) {
+            __syncwarp();
+            t[sl] = qb == pb ? p : prim_pair(A, B, AB2, qb + sl);
+            __syncwarp();
+            const int last = min(SL - 1, pb + sl - qb);
+            if (p.k != 0.0)
+                for (int k = 0; k <= last; k++) {
+                    const PrimPair q = t[k];
+                    if (q.k != 0.0)
+                        quartet_add<LM, LE, LM, LE>(p, Ac, AB, q, AB, qb + k < pb + sl ? 2.0 : 1.0, acc);
+                }
+        }
+    }
     double diag[dM * dN];
     double mx = 0.0;
-    for (int a = 0; a < dM; a++)
-        for (int b = 0; b < dN; b++) {
-            int le[4];
-            double lw[4];
-            int nl = hrr_leaves(c_comp[baseA + a][0], c_comp[baseA + a][1], c_comp[baseA + a][2],
-                                c_comp[baseB + b][0], c_comp[baseB + b][1], c_comp[baseB + b][2], AB, le, lw);
+    sfor<dM>([&](auto ia) {
+        sfor<dN>([&](auto ib) {
+            constexpr int a = decltype(ia)::value, b = decltype(ib)::value;
             double v = 0.0;
-            for (int x = 0; x < nl; x++)
-                for (int y = 0; y < nl; y++) v += lw[x] * lw[y] * acc[(le[x] - eoff) * NEa + (le[y] - eoff)];
+            for_leaves<LM, a, LN, b>(AB, [&](auto e, double we) {
+                double r = 0.0;
+                for_leaves<LM, a, LN, b>(AB, [&](auto f, double wf) {
+                    r += wf * acc[(decltype(e)::value - E0) * NE + decltype(f)::value - E0];
+                });
+                v += we * r;
+            });
+            for (int o = 1; o < SL; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             v = fabs(v);
             diag[a * dN + b] = v;
             mx = fmax(mx, v);
-        }
+        });
+    });
+    if (sl > 0 || g >= npair) return;
     const int bfM = sh.bfoff[M], bfN = sh.bfoff[N];
-    for (int iM = 0; iM < dM; iM++)
-        for (int iN = 0; iN < dN; iN++) bf_scr[(size_t) (bfM + iM) * nbf + bfN + iN] = diag[iN * dM + iM];
+    sfor<dM>([&](auto ia) {
+        sfor<dN>([&](auto ib) {
+            constexpr int i = decltype(ia)::value, j = decltype(ib)::value;
+            constexpr int k2 = i * dN + j;      // position of (N, M)'s element in its own [dN][dM] diagonal
+            bf_scr[(size_t) (bfM + i) * nbf + bfN + j] = diag[j * dM + i];
+            if (M != N) bf_scr[(size_t) (bfN + j) * nbf + bfM + i] = diag[(k2 % dM) * dN + k2 / dM];
+        });
+    });
     sp_scr[M * sh.nsh + N] = mx;
+    sp_scr[N * sh.nsh + M] = mx;
 }
 
-template <int LM>
-static void launch_schwarz_row(const DevShells &sh, const int *ids, const int *start, double *sp, double *bf, int nbf,
-                               cudaStream_t s)
+// Lanes per shell pair: contracted s shells fill a warp with primitive pairs,
+// the d classes have few.
+template <int LM, int LN>
+static void launch_schwarz_class(const DevShells &sh, const int *ids, const int *start, double *sp, double *bf,
+                                 int nbf, Fork &f)
 {
-    for (int ln = 0; ln <= MAX_L_ORB; ln++) {
-        int m0 = start[LM], nM = start[LM + 1] - m0, n0 = start[ln], nN = start[ln + 1] - n0;
-        long long n = (long long) nM * nN;
-        if (n == 0) continue;
-        int blocks = (int) ((n + 63) / 64);
-        switch (ln) {
-        case 0: k_schwarz<LM, 0><<<blocks, 64, 0, s>>>(sh, ids + m0, nM, ids + n0, nN, sp, bf, nbf); break;
-        case 1: k_schwarz<LM, 1><<<blocks, 64, 0, s>>>(sh, ids + m0, nM, ids + n0, nN, sp, bf, nbf); break;
-        case 2: k_schwarz<LM, 2><<<blocks, 64, 0, s>>>(sh, ids + m0, nM, ids + n0, nN, sp, bf, nbf); break;
-        }
-    }
+    const int m0 = start[LM], nM = start[LM + 1] - m0, n0 = start[LN], nN = start[LN + 1] - n0;
+    const long long n = LM == LN ? (long long) nM * (nM + 1) / 2 : (long long) nM * nN;
+    if (n == 0) return;
+    constexpr int SL = LN == 2 ? 1 : (LM + LN >= 3 ? 2 : (LM + LN == 2 ? 8 : 32));
+    const int blocks = (int) ((n * SL + INT_THREADS - 1) / INT_THREADS);
+    k_schwarz<LM, LN><<<blocks, INT_THREADS, 0, f.next()>>>(sh, ids + m0, nM, ids + n0, nN, sp, bf, nbf, SL);
 }
 
 void launch_schwarz_grouped(const DevShells &sh, const int *d_ids, const int *h_start, double *d_sp, double *d_bf,
                             int nbf, cudaStream_t s)
 {
-    launch_schwarz_row<0>(sh, d_ids, h_start, d_sp, d_bf, nbf, s);
-    launch_schwarz_row<1>(sh, d_ids, h_start, d_sp, d_bf, nbf, s);
-    launch_schwarz_row<2>(sh, d_ids, h_start, d_sp, d_bf, nbf, s);
+    Fork f(s, true);
+    launch_schwarz_class<0, 0>(sh, d_ids, h_start, d_sp, d_bf, nbf, f);
+    launch_schwarz_class<1, 0>(sh, d_ids, h_start, d_sp, d_bf, nbf, f);
+    launch_schwarz_class<1, 1>(sh, d_ids, h_start, d_sp, d_bf, nbf, f);
+    launch_schwarz_class<2, 0>(sh, d_ids, h_start, d_sp, d_bf, nbf, f);
+    launch_schwarz_class<2, 1>(sh, d_ids, h_start, d_sp, d_bf, nbf, f);
+    launch_schwarz_class<2, 2>(sh, d_ids, h_start, d_sp, d_bf, nbf, f);
 }
 
 
@@ -707,7 +953,7 @@ __global__ void __launch_bounds__(64) k_one_electron(DevShells sh, const int *id
 
 template <int LM>
 static void launch_1e_row(const DevShells &sh, const int *ids, const int *start, int natoms, const double *Z,
-                          const double *xyz, double *S, double *H, int nbf, cudaStream_t s)
+                          const double *xyz, double *S, double *H, int nbf, Fork &f)
 {
     for (int ln = LM; ln <= MAX_L_ORB; ln++) {   // classes (LM, LN >= LM); the kernel mirrors each block
         int m0 = start[LM], nM = start[LM + 1] - m0, n0 = start[ln], nN = start[ln + 1] - n0;
@@ -715,9 +961,9 @@ static void launch_1e_row(const DevShells &sh, const int *ids, const int *start,
         if (n == 0) continue;
         int blocks = (int) ((n + 63) / 64);
         switch (ln) {
-        case 0: k_one_electron<LM, 0><<<blocks, 64, 0, s>>>(sh, ids + m0, nM, ids + n0, nN, natoms, Z, xyz, S, H, nbf); break;
-        case 1: k_one_electron<LM, 1><<<blocks, 64, 0, s>>>(sh, ids + m0, nM, ids + n0, nN, natoms, Z, xyz, S, H, nbf); break;
-        case 2: k_one_electron<LM, 2><<<blocks, 64, 0, s>>>(sh, ids + m0, nM, ids + n0, nN, natoms, Z, xyz, S, H, nbf); break;
+        case 0: k_one_electron<LM, 0><<<blocks, 64, 0, f.next()>>>(sh, ids + m0, nM, ids + n0, nN, natoms, Z, xyz, S, H, nbf); break;
+        case 1: k_one_electron<LM, 1><<<blocks, 64, 0, f.next()>>>(sh, ids + m0, nM, ids + n0, nN, natoms, Z, xyz, S, H, nbf); break;
+        case 2: k_one_electron<LM, 2><<<blocks, 64, 0, f.next()>>>(sh, ids + m0, nM, ids + n0, nN, natoms, Z, xyz, S, H, nbf); break;
         }
     }
 }
@@ -726,9 +972,10 @@ void launch_one_electron_grouped(const DevShells &sh, const int *d_ids, const in
                                  const double *d_Z, const double *d_xyz, double *d_S, double *d_H, int nbf,
                                  cudaStream_t s)
 {
-    launch_1e_row<0>(sh, d_ids, h_start, natoms, d_Z, d_xyz, d_S, d_H, nbf, s);
-    launch_1e_row<1>(sh, d_ids, h_start, natoms, d_Z, d_xyz, d_S, d_H, nbf, s);
-    launch_1e_row<2>(sh, d_ids, h_start, natoms, d_Z, d_xyz, d_S, d_H, nbf, s);
+    Fork f(s, true);
+    launch_1e_row<0>(sh, d_ids, h_start, natoms, d_Z, d_xyz, d_S, d_H, nbf, f);
+    launch_1e_row<1>(sh, d_ids, h_start, natoms, d_Z, d_xyz, d_S, d_H, nbf, f);
+    launch_1e_row<2>(sh, d_ids, h_start, natoms, d_Z, d_xyz, d_S, d_H, nbf, f);
 }
 
 
