@@ -28,6 +28,8 @@
 #include <cstdio>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "tiles.cuh"
 #include "tscf_internal.h"
 
@@ -382,6 +384,454 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_sytrd_panel(TrdArgs a)
     }
 }
 
+// The same panel for n <= TRC_MAX_N in one thread-block cluster. CTA g owns
+// rows 64 g .. 64 g + 63, as CTA g of k_sytrd_panel does; the rows of the
+// symmetric product are dealt to the CTAs cyclically. The steps' column, norm
+// and dot partials, products and the next row of V and W go to the shared
+// memory of the CTAs that read them (remote stores), followed by a hardware
+// cluster barrier: three barriers a column and no round trips through L2, where
+// the grid's barriers and gathers take 9.7 us a column however small n is: here
+// 5.6 us at n = 260 and 3.3 us at n = 24. A CTA's rows of the trailing matrix
+// stay in shared memory for the panel, which bounds the panels that run here
+// (trc_in_smem).
+// What is left is the chain of dependent FP64 operations of a column step, so
+// sums that others wait for are short trees of adds over shared values instead
+// of shuffles. Every sum has the order of k_sytrd_panel (8 lanes a row, 4 rows a
+// warp, 16 warps a CTA, then CTAs in lane order; levels that only add zeros are
+// left out): the results are the same bit for bit.
+constexpr int TRC_MAX_N = 1024;             // 16 CTAs of 64 rows
+constexpr size_t TRC_SMEM_ROWS = 190 << 10; // most bytes of trailing-matrix rows kept per CTA
+constexpr int TRC_W = TRD_THREADS / 32;     // warps per CTA
+
+// Address of a shared variable in CTA `rank` of the cluster, and a store to it.
+__device__ __forceinline__ unsigned cl_addr(const void *p, int rank)
+{
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned) __cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cl_store(unsigned addr, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+
+// Sum of v[k] over the warp for each k < K (K a power of two, at most 32), in the
+// pairing of a shfl_down tree from 16 to 1: while values are left to split, lanes
+// keep one half of them and hand over the other, so K sums take ~K shuffles
+// instead of 5 K. The sum of value k lands in lane trc_lane<K>(k).
+template <int K>
+__device__ __forceinline__ int trc_lane(int k)
+{
+    int lane = 0, half = K / 2;
+    for (int o = 16; half > 0; o >>= 1, half >>= 1)
+        if (k & half) lane |= o;
+    return lane;
+}
+template <int K>
+__device__ __forceinline__ double warp_sums(double (&v)[K], int lane)
+{
+#pragma unroll
+    for (int o = 16, half = K / 2; o > 0; o >>= 1, half >>= 1) {
+        if (half > 0) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int k = 0; k < half; k++) {
+                const double give = up ? v[k] : v[k + half], keep = up ? v[k + half] : v[k];
+                v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+
+// x[0] + ... + x[15] (stride st) in the pairing of a shfl_down tree.
+__device__ __forceinline__ double tree16(const double *x, int st)
+{
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = x[k * st] + x[(k + 8) * st];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < o; k++) v[k] += v[k + o];
+    return v[0];
+}
+
+constexpr int TRC_LD = TRC_W + 1;   // row pitch of the warp partials: lanes read them a row apart
+// Sum of the warp partials x[cta][warp] of the whole cluster, in every lane.
+__device__ __forceinline__ double cluster_sum(const double (*x)[TRC_LD], int CS, int lane)
+{
+    double v = lane < CS ? tree16(x[lane], 1) : 0.0;
+    for (int o = 8; o > 0; o >>= 1)
+        if (o < CS) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// doubles of the column buffer: whole segments
+__host__ __device__ constexpr int trc_col(int n) { return (n + TRD_SEG - 1) / TRD_SEG * TRD_SEG; }
+
+template <int NSEG>
+__global__ void __launch_bounds__(TRD_THREADS, 1) k_sytrd_cluster(TrdArgs a)
+{
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) double dyn[];
+    __shared__ double s_wv[TRD_NB], s_vv[TRD_NB], s_row[2 * TRD_NB], s_dot[TRC_W][2 * TRD_NB];
+    __shared__ double s_tau[TRD_NB], s_e[TRD_NB], s_d[TRD_NB], s_scal, s_a2;
+    // written by the CTAs of the cluster
+    __shared__ double g_w[16][TRC_LD], g_dot[16][2 * TRD_NB], g_row[2 * TRD_NB], g_y[NSEG][64];
+    cg::cluster_group cl = cg::this_cluster();
+    auto sync_all = [&]() {
+        if (a.G == 1) __syncthreads();
+        else cl.sync();
+    };
+    const int n = a.n, p = a.p, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int CS = a.G, me = blockIdx.x, rbase = 64 * me;
+    double *g_col = dyn, *sA = dyn + trc_col(n);   // the column; this CTA's rows of the trailing matrix
+    const int l8 = lane & 7, r = rbase + (tid >> 3);
+    const bool own = r < n;
+    const int wrow = rbase + 4 * wid;      // first of this warp's four rows
+    constexpr int NQ = TRD_NB / 8;
+    double pv[NQ], pw[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) pv[q] = pw[q] = 0.0;
+    const double *A = a.A;
+    // rows p + me, p + me + CS, ... of the trailing matrix are this CTA's
+    const int c0 = p & ~31, ld = n - c0;   // columns c0..n-1 are kept: whole 32-column blocks from the panel's on
+    for (int k = wid; p + me + k * CS < n; k += TRC_W) {
+        const double *src = A + (size_t) (p + me + k * CS) * n + c0;
+        for (int c = lane; c < ld; c += 32) sA[k * ld + c] = src[c];
+    }
+    for (int l = tid; l < 16 * TRC_LD; l += TRD_THREADS) (&g_w[0][0])[l] = 0.0;
+    for (int l = tid; l < trc_col(n); l += TRD_THREADS) g_col[l] = 0.0;
+    if (tid < 2 * TRD_NB) g_row[tid] = s_row[tid] = 0.0;
+    for (int l = tid; l < TRC_W * 2 * TRD_NB; l += TRD_THREADS) (&s_dot[0][0])[l] = 0.0;
+    if (tid < TRD_NB) s_wv[tid] = s_vv[tid] = 0.0;
+    const unsigned to_col[2] = {cl_addr(g_col + r, min(l8, CS - 1)), cl_addr(g_col + r, min(l8 + 8, CS - 1))};
+    const unsigned to_w = cl_addr(&g_w[me][wid], min(lane, CS - 1));
+    double arow = (own && r >= p) ? A[(size_t) p * n + r] : 0.0;
+    double a2 = 0.0;                       // of the previous column
+    sync_all();   // every CTA runs, its partials zeroed, before the first remote store
+    for (int c = 0; c < a.cols; c++) {
+        const int j = p + c;
+        // ---- phase 1: column j of the panel-corrected matrix, rows j..n-1 (g_row: row j's V and W; W's
+        // entry of the last column still lacks its a2 v)
+        if (wrow < n && wrow + 3 >= j) {
+            double v = l8 == 0 ? arow : 0.0;
+#pragma unroll
+            for (int q = 0; q < NQ; q++) {   // columns behind c - 1 hold zeros
+                const int cc = l8 + 8 * q;
+                const double vj = g_row[cc], w0 = g_row[TRD_NB + cc];
+                const double wj = cc == c - 1 ? w0 + a2 * vj : w0;
+                v -= pv[q] * wj + pw[q] * vj;
+            }
+            v += __shfl_xor_sync(0xffffffff, v, 1);
+            v += __shfl_xor_sync(0xffffffff, v, 2);
+            v += __shfl_xor_sync(0xffffffff, v, 4);
+            if (own && r >= j) {
+                if (l8 < CS) cl_store(to_col[0], v);
+                if (l8 + 8 < CS) cl_store(to_col[1], v);
+            }
+        }
+        sync_all();
+        if (j == n - 1) {
+            if (tid == 0) s_d[c] = g_col[j];
+            break;
+        }
+        // ---- phase 2: the reflector (every CTA forms the same one), y = A v, panel dots
+        if (wid == 0) {
+            // |x|^2 of rows j+2.. in the groups' order: 4 rows, 16 of those, then the 64-row groups in lane order
+            constexpr int H = 2 * NSEG;   // lanes 0-15: group 2 h, lanes 16-31: group 2 h + 1
+            double part[H];
+#pragma unroll
+            for (int h = 0; h < H; h++) {
+                const int rr = 128 * h + 4 * lane;   // the buffer is zero behind the column
+                const double2 u = *reinterpret_cast<const double2 *>(g_col + rr);
+                const double2 v = *reinterpret_cast<const double2 *>(g_col + rr + 2);
+                const double x0 = rr >= j + 2 ? __dmul_rn(u.x, u.x) : 0.0, x1 = rr + 1 >= j + 2 ? __dmul_rn(u.y, u.y) : 0.0;
+                const double x2 = rr + 2 >= j + 2 ? __dmul_rn(v.x, v.x) : 0.0;
+                const double x3 = rr + 3 >= j + 2 ? __dmul_rn(v.y, v.y) : 0.0;
+                part[h] = (x0 + x2) + (x1 + x3);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                for (int h = 0; h < H; h++) part[h] += __shfl_xor_sync(0xffffffffu, part[h], o);
+            // the tree over groups 0..15 (zeros behind the last): groups g and g + 8, then + 4, + 2, + 1
+            double s = 0.0;
+#pragma unroll
+            for (int half = 1; half >= 0; half--) {   // even groups first, then the odd ones
+                double g[8];
+#pragma unroll
+                for (int h = 0; h < 8; h++) g[h] = h < H ? __shfl_sync(0xffffffffu, part[h < H ? h : 0], 16 * (1 - half)) : 0.0;
+                const double x = ((g[0] + g[4]) + (g[2] + g[6])) + ((g[1] + g[5]) + (g[3] + g[7]));
+                s = half ? x : s + x;
+            }
+            const double alpha = g_col[j + 1];
+            double tau, beta, scal;
+            if (s == 0.0) {
+                tau = 0.0;
+                beta = alpha;
+                scal = 0.0;
+            } else {
+                const double nrm = sqrt(alpha * alpha + s);
+                beta = alpha >= 0.0 ? -nrm : nrm;
+                tau = (beta - alpha) / beta;
+                scal = 1.0 / (alpha - beta);
+            }
+            if (lane == 0) {
+                s_tau[c] = tau;
+                s_scal = scal;
+                s_d[c] = g_col[j];
+                s_e[c] = beta;
+            }
+        }
+        __syncthreads();
+        const double tau = s_tau[c], scal = s_scal;
+        const double vr_own = (own && r > j) ? (r == j + 1 ? 1.0 : g_col[r] * scal) : 0.0;
+        if (l8 == (c & 7)) {
+#pragma unroll
+            for (int q = 0; q < NQ; q++)
+                if (q == (c >> 3)) pv[q] = vr_own;
+        }
+        if (c > 0 && rbase < n) {
+            // panel dots W^T v and V^T v of this CTA's rows: 4 rows a warp by shuffles, then the warps in order;
+            // the last two warps add them up while the others go on to the product
+            const int w0 = max(0, (j + 1 - rbase) >> 2), w1 = min(TRC_W, (n - rbase + 3) >> 2);   // warps with rows > j
+            if (wid == w0 - 1) s_dot[wid][lane] = s_dot[wid][lane + 32] = 0.0;   // its last row is done
+            if (wid >= w0 && wid < w1) {
+                // lanes without bit 8 keep W^T v, with it V^T v; without bit 16 columns 0..15, with it 16..31
+                const bool hi8 = lane & 8, hi16 = lane & 16;
+                double d[NQ];
+#pragma unroll
+                for (int q = 0; q < NQ; q++) {
+                    const double dw = __dmul_rn(pw[q], vr_own), dv = __dmul_rn(pv[q], vr_own);
+                    d[q] = (hi8 ? dv : dw) + __shfl_xor_sync(0xffffffff, hi8 ? dw : dv, 8);
+                }
+                static_assert(NQ == 4, "two columns per lane after the second exchange");
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    const double x = (hi16 ? d[q + 2] : d[q]) + __shfl_xor_sync(0xffffffff, hi16 ? d[q] : d[q + 2], 16);
+                    s_dot[wid][(hi8 ? TRD_NB : 0) + l8 + 8 * (q + (hi16 ? 2 : 0))] = x;
+                }
+            }
+            if (wid < TRC_W - 2) {
+                asm volatile("bar.arrive 1, %0;" ::"n"(TRD_THREADS) : "memory");
+            } else {
+                asm volatile("bar.sync 1, %0;" ::"n"(TRD_THREADS) : "memory");
+                const int k = tid & 63;
+                double sacc = 0.0, x[TRC_W];
+#pragma unroll
+                for (int w = 0; w < TRC_W; w++) x[w] = s_dot[w][k];   // idle warps hold zeros
+#pragma unroll
+                for (int w = 0; w < TRC_W; w++) sacc += x[w];
+                for (int q = 0; q < CS; q++) cl_store(cl_addr(&g_dot[me][k], q), sacc);
+            }
+        }
+        {
+            // rows p + me + CS (wid + 16 k), k = 0..3, by segments of TRD_SEG columns
+            constexpr int K = NSEG == 3 ? 16 : 4 * NSEG;   // sums of this warp: (segment, k), padded to a power of two
+            const int s0 = (j + 1) / TRD_SEG;
+            double sum[K];
+#pragma unroll
+            for (int k = 0; k < K; k++) sum[k] = 0.0;
+            // rows are dealt in order, so the last row of a warp tells whether it has one behind row j
+            const int most = (n - 1 - p - me) / CS;   // last local row of this CTA
+            const int last = n - 1 - p < me || most < wid ? -1 : p + me + CS * (most - ((most - wid) & (TRC_W - 1)));
+            const bool any = last > j;
+#pragma unroll
+            for (int sg = 0; sg < NSEG; sg++) {
+                if (sg < s0 || !any) continue;
+                double vs[TRD_SEG / 32];
+                unsigned on = 0;   // this lane's columns j+1..n-1
+#pragma unroll
+                for (int x = 0; x < TRD_SEG / 32; x++) {
+                    const int c2 = sg * TRD_SEG + lane + 32 * x;
+                    vs[x] = c2 == j + 1 ? 1.0 : g_col[c2] * scal;
+                    on |= (unsigned) (c2 > j && c2 < n) << x;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int kk = wid + TRC_W * k, rr = p + me + CS * kk;
+                    if (rr <= j || rr >= n) continue;
+                    const double *row = sA + kk * ld - c0 + sg * TRD_SEG + lane;
+                    double acc[TRD_SEG / 32];
+#pragma unroll
+                    for (int x = 0; x < TRD_SEG / 32; x++)
+                        acc[x] = (on >> x) & 1 ? __dmul_rn(row[32 * x], vs[x]) : 0.0;
+                    sum[sg * 4 + k] = ((acc[0] + acc[4]) + (acc[2] + acc[6])) + ((acc[1] + acc[5]) + (acc[3] + acc[7]));
+                }
+            }
+            if (any) {   // uniform over the warp
+                const double y = warp_sums<K>(sum, lane);
+#pragma unroll
+                for (int k = 0; k < 4 * NSEG; k++) {
+                    const int rr = p + me + CS * (wid + TRC_W * (k & 3));
+                    if (lane == trc_lane<K>(k) && rr > j && rr < n)
+                        cl_store(cl_addr(&g_y[k >> 2][rr & 63], rr >> 6), y);
+                }
+            }
+        }
+        sync_all();
+        // ---- phase 3: w = tau (y - V (W^T v) - W (V^T v)) for this row, partial w.v
+        double ypart = 0.0;
+        const int s0 = (j + 1) / TRD_SEG;
+        if (own && r > j)
+            for (int sg = s0 + l8; sg < NSEG; sg += 8) ypart += g_y[sg][r - rbase];
+        if (tid < 64 && (tid & 31) < c) {
+            double x = 0.0;
+            if (CS > 8) {
+                double y[16];
+#pragma unroll
+                for (int q = 0; q < 16; q++) y[q] = q < CS && 64 * q < n ? g_dot[q][tid] : 0.0;
+                x = tree16(y, 1);
+            } else {
+                double y[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) y[q] = q < CS && 64 * q < n ? g_dot[q][tid] : 0.0;
+                x = ((y[0] + y[4]) + (y[2] + y[6])) + ((y[1] + y[5]) + (y[3] + y[7]));
+            }
+            (tid < 32 ? s_wv : s_vv)[tid & 31] = x;
+        }
+        const bool nxt = c + 1 < a.cols;
+        arow = (nxt && own && r >= j + 1) ? A[(size_t) (j + 1) * n + r] : 0.0;
+        __syncthreads();
+        if (wrow < n && wrow + 3 > j) {
+            double t = ypart;
+#pragma unroll
+            for (int q = 0; q < NQ; q++) {
+                // column c itself: W's entry is still zero, V's meets a zero sum
+                const int cc = l8 + 8 * q;
+                t -= pv[q] * s_wv[cc] + pw[q] * s_vv[cc];
+            }
+            t += __shfl_xor_sync(0xffffffff, t, 1);
+            t += __shfl_xor_sync(0xffffffff, t, 2);
+            t += __shfl_xor_sync(0xffffffff, t, 4);
+            const double w = (own && r > j) ? tau * t : 0.0;
+            if (l8 == (c & 7)) {
+#pragma unroll
+                for (int q = 0; q < NQ; q++)
+                    if (q == (c >> 3)) pw[q] = w;
+            }
+            if (nxt && r == j + 1) {   // row j+1's V and W for everyone (W of column c before its a2 v)
+#pragma unroll
+                for (int q = 0; q < NQ; q++) {
+                    s_row[l8 + 8 * q] = pv[q];
+                    s_row[TRD_NB + l8 + 8 * q] = pw[q];
+                }
+            }
+            double wd = __dmul_rn(w, vr_own);   // the same in a row's 8 lanes
+            wd += __shfl_xor_sync(0xffffffff, wd, 16);
+            wd += __shfl_xor_sync(0xffffffff, wd, 8);
+            if (lane < CS) cl_store(to_w, wd);
+        } else if (wrow < n && wrow + 3 == j) {   // these rows are done
+            if (lane < CS) cl_store(to_w, 0.0);
+        }
+        if (nxt && me == (j + 1) / 64) {
+            __syncthreads();
+            const double x = s_row[tid & 63];
+            for (int q = tid >> 6; q < CS; q += TRD_THREADS / 64) cl_store(cl_addr(&g_row[tid & 63], q), x);
+        }
+        sync_all();
+        // ---- phase 4: a2 = -tau/2 (w.v), w += a2 v
+        if (wid == 0) {
+            const double x = -0.5 * tau * cluster_sum(g_w, CS, lane);
+            if (lane == 0) s_a2 = x;
+        }
+        __syncthreads();
+        a2 = s_a2;
+        if (l8 == (c & 7)) {
+#pragma unroll
+            for (int q = 0; q < NQ; q++)
+                if (q == (c >> 3)) pw[q] += a2 * pv[q];
+        }
+    }
+    // the reflectors, and the final W of the rows behind the panel, into both stacked panels (nothing is written
+    // to global memory inside the loop: a barrier's release would wait for it)
+    if (own) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const int cc = l8 + 8 * q;
+            if (cc < a.cols && r > p + cc) {
+                a.VT[(size_t) (p + cc) * n + r] = pv[q];
+                a.PVW[(size_t) cc * n + r] = pv[q];
+                a.PWV[(size_t) (TRD_NB + cc) * n + r] = pv[q];
+            }
+            if (cc < a.cols && r >= p + a.cols) {
+                a.PWV[(size_t) cc * n + r] = pw[q];
+                a.PVW[(size_t) (TRD_NB + cc) * n + r] = pw[q];
+            }
+        }
+    }
+    if (me == 0 && tid < a.cols) {
+        a.d[p + tid] = s_d[tid];
+        if (p + tid < n - 1) {
+            a.e[p + tid] = s_e[tid];
+            a.tau[p + tid] = s_tau[tid];
+        }
+    }
+    sync_all();   // no CTA leaves while another may still write to it
+}
+
+// CTAs of the cluster: every 64 rows need an owner; up to 16, about 24 rows of the product each.
+int trc_ctas(int n) { return n <= 64 ? 1 : std::min(16, std::max((n + 63) / 64, (n + 23) / 24)); }
+// Bytes of a CTA's rows of the trailing matrix of size m (with the panel's leading partial column block).
+size_t trc_rows_bytes(int n, int m) { return sizeof(double) * (size_t) ((m + trc_ctas(n) - 1) / trc_ctas(n)) * (m + 31); }
+// The panels that run in a cluster: those whose trailing rows fit in its shared memory (616 rows on 16 CTAs).
+// Larger ones would stream A from L2 into 16 SMs: 16.6 us a column at 1010 rows against 10.4 us on the whole chip.
+bool trc_in_smem(int n, int m) { return trc_rows_bytes(n, m) <= TRC_SMEM_ROWS; }
+size_t trc_smem(int n, int m) { return sizeof(double) * (size_t) trc_col(n) + trc_rows_bytes(n, m); }
+
+const void *trc_kernel(int n)
+{
+    switch ((n + TRD_SEG - 1) / TRD_SEG) {
+    case 1: return (const void *) k_sytrd_cluster<1>;
+    case 2: return (const void *) k_sytrd_cluster<2>;
+    case 3: return (const void *) k_sytrd_cluster<3>;
+    default: return (const void *) k_sytrd_cluster<4>;
+    }
+}
+
+// Launch configuration of the cluster panel with m trailing rows; attr must outlive it.
+cudaLaunchConfig_t trc_config(int n, int m, cudaStream_t s, cudaLaunchAttribute *attr)
+{
+    const unsigned cs = trc_ctas(n);
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = cs;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs);
+    cfg.blockDim = dim3(TRD_THREADS);
+    cfg.dynamicSmemBytes = trc_smem(n, m);
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Whether the device takes the cluster panel for n rows.
+bool trc_usable(int n)
+{
+    if (n > TRC_MAX_N) return false;
+    const void *k = trc_kernel(n);
+    const int most = (int) (sizeof(double) * trc_col(n) + TRC_SMEM_ROWS);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = trc_config(n, n, 0, &attr);
+    cfg.dynamicSmemBytes = most;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 // Partial Gram matrices V_B^T V_B of the reflector blocks (the reflectors of
 // block B are rows p0..p0+bb-1 of VT, zero before column p0 + 1): CTA (B,
 // 32 x 32 tile, slice ks of the columns) writes its slice's sum to Gp[B][ks].
@@ -423,35 +873,64 @@ __global__ void __launch_bounds__(256) k_wy_gram(const double *VT, double *Gp, i
 // T of the compact WY form of each block of BT_NB reflectors:
 // H_p0 ... H_(p0+bb-1) = I - V T V^T, T upper triangular (LAPACK dlarft,
 // forward, columnwise), from the block's Gram matrix (the sum of its
-// GR_KS slices). One CTA per block.
-__global__ void __launch_bounds__(256) k_wy_tfactor(const double *Gp, const double *tau, double *Tf, int nref)
+// GR_KS slices). One CTA per block, one warp per four rows of T: row i needs
+// only its own entries, T(i, c) = -tau_c sum_(l = i..c-1) T(i, l) G(l, c), so a
+// warp runs along its row and adds T(i, l) G(l, c) to every later column c (lane
+// c % 32) as soon as T(i, l) is known. The sums run over l in the order of the
+// column-by-column form, which one thread per row ran as a serial chain of
+// bb^2 / 2 dependent multiply-adds: 280 us per call, whatever n, now 50 us
+// (most of it the Gram slices' sum).
+constexpr int TF_THREADS = 1024, TF_ROWS = BT_NB / (TF_THREADS / 32);
+__global__ void __launch_bounds__(TF_THREADS) k_wy_tfactor(const double *Gp, const double *tau, double *Tf, int nref)
 {
-    extern __shared__ double tsm[];
-    constexpr int LD = BT_NB + 1;
-    double *T = tsm;                       // BT_NB x LD
-    double *Gc = tsm + BT_NB * LD;         // column c of the Gram matrix
-    const int B = blockIdx.x, p0 = B * BT_NB, bb = min(BT_NB, nref - p0), tid = threadIdx.x;
+    extern __shared__ double tsm[];        // the Gram matrix, BT_NB x BT_NB
+    constexpr int NC = BT_NB / 32;
+    const int B = blockIdx.x, p0 = B * BT_NB, bb = min(BT_NB, nref - p0), tid = threadIdx.x, lane = tid & 31;
     const double *G = Gp + (size_t) B * GR_KS * BT_NB * BT_NB;
-    for (int l = tid; l < BT_NB * LD; l += blockDim.x) T[l] = 0.0;
-    __syncthreads();
-    for (int c = 0; c < bb; c++) {
-        const double tc = tau[p0 + c];
-        if (tid < c) {
-            double g = 0.0;
-            for (int ks = 0; ks < GR_KS; ks++) g += G[(size_t) ks * BT_NB * BT_NB + (size_t) tid * BT_NB + c];
-            Gc[tid] = g;
-        }
-        __syncthreads();
-        if (tid < c) {
-            double sacc = 0.0;
-            for (int l = tid; l < c; l++) sacc += T[tid * LD + l] * Gc[l];
-            T[tid * LD + c] = -tc * sacc;
-        }
-        if (tid == 0) T[c * LD + c] = tc;
-        __syncthreads();
+    for (int l = tid; l < BT_NB * BT_NB; l += TF_THREADS) {
+        double g = 0.0;
+#pragma unroll
+        for (int ks = 0; ks < GR_KS; ks++) g += G[(size_t) ks * BT_NB * BT_NB + l];
+        tsm[l] = g;
     }
-    for (int l = tid; l < BT_NB * BT_NB; l += blockDim.x)
-        Tf[(size_t) B * BT_NB * BT_NB + l] = T[(l / BT_NB) * LD + l % BT_NB];
+    double tc[NC];
+#pragma unroll
+    for (int q = 0; q < NC; q++) tc[q] = lane + 32 * q < bb ? tau[p0 + lane + 32 * q] : 0.0;
+    __syncthreads();
+    double acc[TF_ROWS][NC], t[TF_ROWS][NC];
+    const int i0 = tid >> 5;               // rows i0, i0 + 32, ...
+#pragma unroll
+    for (int x = 0; x < TF_ROWS; x++)
+#pragma unroll
+        for (int q = 0; q < NC; q++) acc[x][q] = t[x][q] = 0.0;
+#pragma unroll
+    for (int lq = 0; lq < NC; lq++) {
+        for (int ll = 0; ll < 32; ll++) {
+            const int l = 32 * lq + ll;
+            if (l < i0) continue;
+            if (l >= bb) break;
+            double g[NC];
+#pragma unroll
+            for (int q = lq; q < NC; q++) g[q] = tsm[l * BT_NB + lane + 32 * q];
+#pragma unroll
+            for (int x = 0; x < TF_ROWS; x++) {
+                const int i = i0 + 32 * x;
+                if (l < i) continue;
+                // lane ll holds column l: its sum is complete
+                const double mine = l == i ? tc[lq] : -tc[lq] * acc[x][lq];
+                if (lane == ll) t[x][lq] = mine;
+                const double tl = __shfl_sync(0xffffffffu, mine, ll);
+#pragma unroll
+                for (int q = lq; q < NC; q++)
+                    if (lane + 32 * q > l) acc[x][q] = fma(tl, g[q], acc[x][q]);
+            }
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < TF_ROWS; x++)
+#pragma unroll
+        for (int q = 0; q < NC; q++)
+            Tf[(size_t) B * BT_NB * BT_NB + (size_t) (i0 + 32 * x) * BT_NB + lane + 32 * q] = t[x][q];
 }
 
 // ------------------------------------------------------------------ divide and conquer
@@ -958,6 +1437,7 @@ __global__ void k_hash_fill(double *A, size_t n)
 // ------------------------------------------------------------------ host side
 struct Eig {
     int n = 0, G = 1, npanels = 0, nblk = 0;
+    bool cluster = false;   // panels in one thread-block cluster (k_sytrd_cluster)
     // tridiagonalisation and back-transformation
     double *A = nullptr, *VT = nullptr, *PVW = nullptr, *PWV = nullptr, *d = nullptr, *e = nullptr, *tau = nullptr,
            *col = nullptr, *y = nullptr, *part = nullptr, *Gb = nullptr, *Tf = nullptr, *Y = nullptr, *Y2 = nullptr;
@@ -1121,6 +1601,7 @@ Eig *eig_create(int n, cudaStream_t s)
         delete E;
         return nullptr;
     }
+    E->cluster = trc_usable(n);
     E->npanels = (n + TRD_NB - 1) / TRD_NB;
     E->nblk = (n - 1 + BT_NB - 1) / BT_NB;   // blocks of the n - 1 reflectors
     const size_t nn = (size_t) n * n;
@@ -1206,8 +1687,16 @@ int tridiagonalize(Eig *E, const double *d_A, cudaStream_t s)
         void *args[] = {&a};
         g_launches++;
         g_eig_launches++;
-        TSCF_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *) k_sytrd_panel, dim3(E->G), dim3(TRD_THREADS), args,
-                                                    dyn, s));
+        const int m = n - a.p;
+        if (E->cluster && trc_in_smem(n, m)) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = trc_config(n, m, s, &attr);
+            a.G = (int) cfg.gridDim.x;
+            TSCF_CUDA_CHECK(cudaLaunchKernelExC(&cfg, trc_kernel(n), args));
+        } else {
+            TSCF_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *) k_sytrd_panel, dim3(E->G), dim3(TRD_THREADS),
+                                                        args, dyn, s));
+        }
         const int q = a.p + a.cols, mt = n - q;
         if (mt > 0) {
             // A22 -= V W^T + W V^T = PVW^T PWV over the trailing columns (a full panel: cols = TRD_NB)
@@ -1260,7 +1749,7 @@ int back_transform(Eig *E, const double *Zc, double *d_V, cudaStream_t s)
     g_launches += 3;
     g_eig_launches += 3;
     k_wy_gram<<<dim3(E->nblk, (BT_NB / 32) * (BT_NB / 32), GR_KS), 256, 0, s>>>(E->VT, E->Gb, n, nref);
-    k_wy_tfactor<<<E->nblk, 256, sizeof(double) * (BT_NB * (BT_NB + 1) + BT_NB), s>>>(E->Gb, E->tau, E->Tf, nref);
+    k_wy_tfactor<<<E->nblk, TF_THREADS, sizeof(double) * BT_NB * BT_NB, s>>>(E->Gb, E->tau, E->Tf, nref);
     k_transpose<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, s>>>(Zc, d_V, n);
     for (int B = E->nblk - 1; B >= 0; B--) {
         const int p0 = B * BT_NB, bb = std::min(BT_NB, nref - p0), mv = n - p0 - 1;
