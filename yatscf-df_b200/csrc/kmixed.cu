@@ -1185,14 +1185,18 @@ static void kmix_prepare(KMix *k, const double *Cocc, const double *S, cudaStrea
     // align C_n to C_{n-1}: R = polar(C_n^T S C_{n-1}) by Newton-Schulz; R = I if it does not converge
     dgemm(false, false, n, o, n, 1.0, S, n, k->Cprev, o, 0.0, k->SC, o, s);
     dgemm(true, false, o, o, n, 1.0, Cocc, o, k->SC, o, 0.0, k->X, o, s);
-    for (int it = 0; it < 12; it++) {
+    if (ns_fits(o)) {
+        ns_polar(k->X, k->Y, o, 12, s);
+    } else {
+        for (int it = 0; it < 12; it++) {
+            dgemm(true, false, o, o, o, 1.0, k->X, o, k->X, o, 0.0, k->Y, o, s);
+            k_ns_z<<<(o * o + 255) / 256, 256, 0, s>>>(k->Y, k->Z, o);
+            dgemm(false, false, o, o, o, 1.0, k->X, o, k->Z, o, 0.0, k->M, o, s);
+            std::swap(k->X, k->M);
+            g_launches++;
+        }
         dgemm(true, false, o, o, o, 1.0, k->X, o, k->X, o, 0.0, k->Y, o, s);
-        k_ns_z<<<(o * o + 255) / 256, 256, 0, s>>>(k->Y, k->Z, o);
-        dgemm(false, false, o, o, o, 1.0, k->X, o, k->Z, o, 0.0, k->M, o, s);
-        std::swap(k->X, k->M);
-        g_launches++;
     }
-    dgemm(true, false, o, o, o, 1.0, k->X, o, k->X, o, 0.0, k->Y, o, s);
     k_select_r<<<1, 1024, 0, s>>>(k->X, k->Y, k->R, o, 1e-12);
     dgemm(false, false, n, o, o, 1.0, Cocc, o, k->R, o, 0.0, k->Cal, o, s);
     const size_t nc = (size_t) n * o;

@@ -213,6 +213,207 @@ static void dgemm_variant(int v, bool ta, bool tb, int m, int n, int k, double a
     else dgemm_shape<64, 64>(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s);
 }
 
+// ------------------------------------------------------------------ small products
+// C = alpha op(A) op(B) for products too small to be worth tuning (m n k < 2e6):
+// one output per thread in 16 x 16 tiles, K in chunks of 64 that are loaded one
+// chunk ahead. They are latency-bound, and the 64 x 64 tile gives one of them
+// a handful of CTAs with 16 outputs per thread and a barrier pair every 16 steps: a
+// 60 x 60 x 60 product took 9.1 us, now 3.0 us. Each output is the same chain of
+// multiply-adds over k, bit for bit.
+constexpr int SM_T = 16, SM_K = 64;
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(256) k_dgemm_small(int m, int n, int k, double alpha, const double *__restrict__ A,
+                                                     int lda, const double *__restrict__ B, int ldb, double *C, int ldc)
+{
+    __shared__ double As[2][SM_K][SM_T + 1], Bs[2][SM_K][SM_T + 1];
+    constexpr int NL = SM_K * SM_T / 256;
+    const int tid = threadIdx.x, tx = tid % SM_T, ty = tid / SM_T;
+    const int m0 = blockIdx.y * SM_T, n0 = blockIdx.x * SM_T;
+    double ra[NL], rb[NL];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int r = 0; r < NL; r++) {
+            const int l = tid + 256 * r;
+            const int ak = TA ? l / SM_T : l % SM_K, ar = TA ? l % SM_T : l / SM_K;
+            const int bk = TB ? l % SM_K : l / SM_T, bc = TB ? l / SM_K : l % SM_T;
+            const int gi = m0 + ar, gj = n0 + bc;
+            ra[r] = (gi < m && k0 + ak < k) ? (TA ? A[(size_t) (k0 + ak) * lda + gi] : A[(size_t) gi * lda + k0 + ak]) : 0.0;
+            rb[r] = (gj < n && k0 + bk < k) ? (TB ? B[(size_t) gj * ldb + k0 + bk] : B[(size_t) (k0 + bk) * ldb + gj]) : 0.0;
+        }
+    };
+    load(0);
+    double acc = 0.0;
+    for (int k0 = 0, buf = 0; k0 < k; k0 += SM_K, buf ^= 1) {
+#pragma unroll
+        for (int r = 0; r < NL; r++) {
+            const int l = tid + 256 * r;
+            As[buf][TA ? l / SM_T : l % SM_K][TA ? l % SM_T : l / SM_K] = ra[r];
+            Bs[buf][TB ? l % SM_K : l / SM_T][TB ? l / SM_K : l % SM_T] = rb[r];
+        }
+        __syncthreads();   // the other buffer's readers have passed the barrier of the chunk before
+        if (k0 + SM_K < k) load(k0 + SM_K);
+        const int kn = min(SM_K, k - k0);
+        int kk = 0;
+        for (; kk + 8 <= kn; kk += 8) {
+#pragma unroll
+            for (int q = 0; q < 8; q++) acc = fma(As[buf][kk + q][ty], Bs[buf][kk + q][tx], acc);
+        }
+        for (; kk < kn; kk++) acc = fma(As[buf][kk][ty], Bs[buf][kk][tx], acc);
+    }
+    if (m0 + ty < m && n0 + tx < n) C[(size_t) (m0 + ty) * ldc + n0 + tx] = alpha * acc;
+}
+
+static void dgemm_small(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda, const double *B,
+                        int ldb, double *C, int ldc, cudaStream_t s)
+{
+    const dim3 grid((n + SM_T - 1) / SM_T, (m + SM_T - 1) / SM_T);
+    g_launches++;
+    if (!ta && !tb) k_dgemm_small<false, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, C, ldc);
+    else if (!ta && tb) k_dgemm_small<false, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, C, ldc);
+    else if (ta && !tb) k_dgemm_small<true, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, C, ldc);
+    else k_dgemm_small<true, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, C, ldc);
+}
+
+// ------------------------------------------------------------------ Newton-Schulz iterations of small matrices
+// The whole iteration of an o x o matrix in one CTA, matrices in shared memory
+// (row pitch NS padded to 4, zeros in the padding): the occupied dimension of a
+// small molecule makes each product a few us of latency, and launching three
+// kernels per step cost more than the step (a water cluster's SCF iteration had
+// 37 + 32 such launches per molecule and refinement step). 4 x 4 outputs per
+// thread; each output is one chain of multiply-adds over k in order, as in
+// dgemm's small products: the same bits.
+constexpr int NS_THREADS = 512;
+constexpr int NS_MAX = 84;   // 4 matrices of 84 x 84 doubles in 227 KB
+
+// C = op(A) B over o terms; op(A)(i, k) = TA ? A[k][i] : A[i][k]; C must not be A or B.
+template <bool TA>
+__device__ __forceinline__ void ns_product(const double *A, const double *B, double *C, int o, int ld)
+{
+    const int nt = ld / 4;
+    for (int t = threadIdx.x; t < nt * nt; t += NS_THREADS) {
+        const int i0 = t / nt * 4, j0 = t % nt * 4;
+        double acc[4][4] = {};
+#pragma unroll 4
+        for (int k = 0; k < o; k++) {
+            double a[4];
+            if (TA) {
+                const double2 u = *reinterpret_cast<const double2 *>(A + k * ld + i0);
+                const double2 v = *reinterpret_cast<const double2 *>(A + k * ld + i0 + 2);
+                a[0] = u.x, a[1] = u.y, a[2] = v.x, a[3] = v.y;
+            } else {
+#pragma unroll
+                for (int x = 0; x < 4; x++) a[x] = A[(i0 + x) * ld + k];
+            }
+            const double2 b0 = *reinterpret_cast<const double2 *>(B + k * ld + j0);
+            const double2 b1 = *reinterpret_cast<const double2 *>(B + k * ld + j0 + 2);
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                acc[x][0] = fma(a[x], b0.x, acc[x][0]);
+                acc[x][1] = fma(a[x], b0.y, acc[x][1]);
+                acc[x][2] = fma(a[x], b1.x, acc[x][2]);
+                acc[x][3] = fma(a[x], b1.y, acc[x][3]);
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            *reinterpret_cast<double2 *>(C + (i0 + x) * ld + j0) = make_double2(acc[x][0], acc[x][1]);
+            *reinterpret_cast<double2 *>(C + (i0 + x) * ld + j0 + 2) = make_double2(acc[x][2], acc[x][3]);
+        }
+    }
+    __syncthreads();
+}
+// M <- 1.5 I - 0.5 M (the padding stays zero)
+__device__ __forceinline__ void ns_flip(double *M, int o, int ld)
+{
+    for (int l = threadIdx.x; l < o * o; l += NS_THREADS) {
+        const int i = l / o, j = l - i * o;
+        M[i * ld + j] = (i == j ? 1.5 : 0.0) - 0.5 * M[i * ld + j];
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ void ns_load(const double *g, double *M, int o, int ld)
+{
+    for (int l = threadIdx.x; l < ld * ld; l += NS_THREADS) {
+        const int i = l / ld, j = l - i * ld;
+        M[l] = (i < o && j < o) ? g[(size_t) i * o + j] : 0.0;
+    }
+}
+__device__ __forceinline__ void ns_store(const double *M, double *g, int o, int ld)
+{
+    for (int l = threadIdx.x; l < o * o; l += NS_THREADS) g[l] = M[l / o * ld + l % o];
+}
+
+// iters steps X <- X (1.5 I - 0.5 X^T X); X in place, Y = X^T X of the result.
+__global__ void __launch_bounds__(NS_THREADS) k_ns_polar(double *gX, double *gY, int o, int iters)
+{
+    extern __shared__ __align__(16) double ns[];
+    const int ld = (o + 3) & ~3;
+    double *X = ns, *Y = ns + ld * ld, *M = Y + ld * ld;
+    ns_load(gX, X, o, ld);
+    __syncthreads();
+    for (int it = 0; it < iters; it++) {
+        ns_product<true>(X, X, Y, o, ld);
+        ns_flip(Y, o, ld);
+        ns_product<false>(X, Y, M, o, ld);
+        double *t = X;
+        X = M;
+        M = t;
+    }
+    ns_product<true>(X, X, Y, o, ld);
+    ns_store(X, gX, o, ld);
+    ns_store(Y, gY, o, ld);
+}
+
+// Z = M^-1/2 by iters coupled steps T = 1.5 I - 0.5 Z Y, Y <- Y T, Z <- T Z from Y = M, Z = I.
+__global__ void __launch_bounds__(NS_THREADS) k_ns_inv_sqrt(const double *gM, double *gZ, int o, int iters)
+{
+    extern __shared__ __align__(16) double ns[];
+    const int ld = (o + 3) & ~3;
+    double *Y = ns, *Z = Y + ld * ld, *T = Z + ld * ld, *W = T + ld * ld;
+    ns_load(gM, Y, o, ld);
+    for (int l = threadIdx.x; l < ld * ld; l += NS_THREADS) Z[l] = (l / ld == l % ld && l / ld < o) ? 1.0 : 0.0;
+    __syncthreads();
+    for (int it = 0; it < iters; it++) {
+        ns_product<false>(Z, Y, T, o, ld);
+        ns_flip(T, o, ld);
+        ns_product<false>(Y, T, W, o, ld);
+        double *t = Y;
+        Y = W;
+        W = t;
+        ns_product<false>(T, Z, W, o, ld);
+        t = Z;
+        Z = W;
+        W = t;
+    }
+    ns_store(Z, gZ, o, ld);
+}
+
+static size_t ns_smem(int o, int mats)
+{
+    const size_t ld = (o + 3) & ~3;
+    return sizeof(double) * mats * ld * ld;
+}
+
+bool ns_fits(int o) { return o >= 1 && o <= NS_MAX; }
+
+int ns_polar(double *d_X, double *d_Y, int o, int iters, cudaStream_t s)
+{
+    const int bytes = (int) ns_smem(o, 3);
+    TSCF_CUDA_CHECK(cudaFuncSetAttribute(k_ns_polar, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    k_ns_polar<<<1, NS_THREADS, bytes, s>>>(d_X, d_Y, o, iters);
+    g_launches++;
+    return OK;
+}
+
+int ns_inv_sqrt(const double *d_M, double *d_Z, int o, int iters, cudaStream_t s)
+{
+    const int bytes = (int) ns_smem(o, 4);
+    TSCF_CUDA_CHECK(cudaFuncSetAttribute(k_ns_inv_sqrt, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    k_ns_inv_sqrt<<<1, NS_THREADS, bytes, s>>>(d_M, d_Z, o, iters);
+    g_launches++;
+    return OK;
+}
+
 void dgemm(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda, const double *B, int ldb,
            double beta, double *C, int ldc, cudaStream_t s)
 {
@@ -235,6 +436,10 @@ void dgemm(bool ta, bool tb, int m, int n, int k, double alpha, const double *A,
         if (tune_enabled() && cs == cudaStreamCaptureStatusNone && beta == 0.0 && disjoint(A, ea) && disjoint(B, eb) &&
             (double) m * n * k >= 2e6) {
             v = tune_run(key, {0, 1, 2, 3, 4, 5}, [&](int c) { dgemm_variant(c, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s); }, s);
+            return;
+        }
+        if (beta == 0.0 && (double) m * n * k < 2e6) {
+            dgemm_small(ta, tb, m, n, k, alpha, A, lda, B, ldb, C, ldc, s);
             return;
         }
     }

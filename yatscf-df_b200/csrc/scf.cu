@@ -430,6 +430,10 @@ __global__ void k_eye(double *A, int n)
 // M^-1/2 of an SPD matrix close to I (coupled Newton-Schulz), result in Z.
 static void inv_sqrt_ns(const double *M, double *Y, double *Z, double *T, double *W, int o, int iters, cudaStream_t s)
 {
+    if (ns_fits(o)) {
+        ns_inv_sqrt(M, Z, o, iters, s);
+        return;
+    }
     const unsigned nb = (unsigned) ((o * o + 255) / 256);
     cudaMemcpyAsync(Y, M, sizeof(double) * o * o, cudaMemcpyDeviceToDevice, s);
     k_eye<<<nb, 256, 0, s>>>(Z, o);

@@ -123,6 +123,11 @@ void dgemm(bool ta, bool tb, int m, int n, int k, double alpha, const double *A,
 // The same product with the tile picked from the call shape (no tuning run).
 void dgemm_untuned(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda,
                    const double *B, int ldb, double beta, double *C, int ldc, cudaStream_t s);
+// Newton-Schulz iterations of an o x o matrix in one launch where ns_fits(o) (linalg.cu): the polar factor's
+// steps X <- X (1.5 I - 0.5 X^T X) with Y = X^T X of the result, and Z = M^-1/2 of an M close to I.
+bool ns_fits(int o);
+int  ns_polar(double *d_X, double *d_Y, int o, int iters, cudaStream_t s);
+int  ns_inv_sqrt(const double *d_M, double *d_Z, int o, int iters, cudaStream_t s);
 // ERR_CUDA (with a message) when a launch since the last check failed; the error is not cleared.
 int cuda_launch_rc(const char *what);
 // Streaming multiprocessors of the current device (queried once per device).
