@@ -1818,7 +1818,7 @@ int dominant_subspace(Eig *E, const double *d_M, double *d_U, double *d_W, doubl
     if (!E || o <= 0 || o > n || iters < 1) return ERR_INPUT;
     if (E->go < o) {
         if (E->Gx) {
-            cudaFree(E->Gx);
+            dev_free(E->Gx, s);
             E->allocs.erase(std::find(E->allocs.begin(), E->allocs.end(), (void *) E->Gx));
             E->Gx = nullptr;
         }

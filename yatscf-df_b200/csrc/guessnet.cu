@@ -194,24 +194,24 @@ int work_alloc(MlpWork &w, int din, int hid, int dout, int cap)
     const size_t pmax = (size_t) w.splits * std::max((size_t) din * hid, std::max((size_t) hid * hid, (size_t) hid * dout));
     float **fb[] = {&w.Z1, &w.H1, &w.Z2, &w.H2, &w.dH, &w.dH2};
     for (float **b : fb) {
-        if (cudaMalloc(b, sizeof(float) * ch) != cudaSuccess) return ERR_ALLOC;
+        if (dev_malloc((void **) b, sizeof(float) * ch, 0) != OK) return ERR_ALLOC;
         w.mem.push_back(*b);
     }
     float **ob[] = {&w.Y, &w.dY};
     for (float **b : ob) {
-        if (cudaMalloc(b, sizeof(float) * co) != cudaSuccess) return ERR_ALLOC;
+        if (dev_malloc((void **) b, sizeof(float) * co, 0) != OK) return ERR_ALLOC;
         w.mem.push_back(*b);
     }
-    if (cudaMalloc(&w.part, sizeof(float) * pmax) != cudaSuccess) return ERR_ALLOC;
+    if (dev_malloc((void **) &w.part, sizeof(float) * pmax, 0) != OK) return ERR_ALLOC;
     w.mem.push_back(w.part);
-    if (cudaMalloc(&w.loss_part, sizeof(double) * LOSS_BLOCKS) != cudaSuccess) return ERR_ALLOC;
+    if (dev_malloc((void **) &w.loss_part, sizeof(double) * LOSS_BLOCKS, 0) != OK) return ERR_ALLOC;
     w.mem.push_back(w.loss_part);
     return OK;
 }
 
 void work_free(MlpWork &w)
 {
-    for (void *p : w.mem) cudaFree(p);
+    for (void *p : w.mem) dev_free(p, 0);
     w.mem.clear();
 }
 
@@ -374,7 +374,7 @@ int guessnet_load(GuessNet **out, const char *path)
         const size_t np = mlp_param_count(net->din, net->hid, net->dout[t]);
         std::vector<float> h(np + 2 * (size_t) net->dout[t]);
         if (fread(h.data(), sizeof(float), h.size(), f) != h.size()) { rc = ERR_INPUT; break; }
-        if (cudaMalloc(&net->d_params[t], sizeof(float) * h.size()) != cudaSuccess) { rc = ERR_ALLOC; break; }
+        if (dev_malloc((void **) &net->d_params[t], sizeof(float) * h.size(), 0) != OK) { rc = ERR_ALLOC; break; }
         cudaMemcpy(net->d_params[t], h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice);
         net->d_scale[t] = net->d_params[t] + np;
         net->d_offset[t] = net->d_scale[t] + net->dout[t];
@@ -402,7 +402,7 @@ static void work_release(GuessWork *gw)
 {
     if (!gw) return;
     work_free(gw->w);
-    for (void *p : gw->mem) cudaFree(p);
+    for (void *p : gw->mem) dev_free(p, 0);
     gw->mem.clear();
     gw->cap_pairs = gw->cap_rows = 0;
 }
@@ -418,7 +418,7 @@ static int work_reserve(GuessNet *net, int np, int maxrows)
     np = std::max(np, 1);
     maxrows = std::max(maxrows, 1);
     auto dal = [&](void **p, size_t bytes) {
-        if (cudaMalloc(p, bytes ? bytes : 16) != cudaSuccess) return false;
+        if (dev_malloc(p, bytes, 0) != OK) return false;
         gw->mem.push_back(*p);
         return true;
     };
@@ -500,7 +500,7 @@ void guessnet_free(GuessNet *net)
         delete net->work;
     }
     for (int t = 0; t < G_NTYPES; t++)
-        if (net->d_params[t]) cudaFree(net->d_params[t]);
+        dev_free(net->d_params[t], 0);
     delete net;
 }
 
@@ -564,7 +564,7 @@ int guessnet_train(const float *feat, const float *target, const int *type, long
             MlpWork w{};
             std::vector<void *> mem;
             auto dal = [&](void **p, size_t bytes) {
-                if (cudaMalloc(p, bytes) != cudaSuccess) return false;
+                if (dev_malloc(p, bytes, 0) != OK) return false;
                 mem.push_back(*p);
                 return true;
             };
@@ -614,7 +614,7 @@ int guessnet_train(const float *feat, const float *target, const int *type, long
                 if (final_loss) final_loss[t] = (float) last;
             }
             work_free(w);
-            for (void *p : mem) cudaFree(p);
+            for (void *p : mem) dev_free(p, 0);
         } else if (final_loss) {
             final_loss[t] = 0.f;
         }
@@ -643,9 +643,9 @@ int guessnet_grad(int din, int hid, int dout, const float *params, const float *
     float *dp = nullptr, *dX = nullptr, *dT = nullptr, *dg = nullptr;
     MlpWork w{};
     int rc = OK;
-    if (cudaMalloc(&dp, sizeof(float) * np) != cudaSuccess || cudaMalloc(&dg, sizeof(float) * np) != cudaSuccess ||
-        cudaMalloc(&dX, sizeof(float) * (size_t) n * din) != cudaSuccess ||
-        cudaMalloc(&dT, sizeof(float) * (size_t) n * dout) != cudaSuccess)
+    if (dev_malloc((void **) &dp, sizeof(float) * np, 0) != OK || dev_malloc((void **) &dg, sizeof(float) * np, 0) != OK ||
+        dev_malloc((void **) &dX, sizeof(float) * (size_t) n * din, 0) != OK ||
+        dev_malloc((void **) &dT, sizeof(float) * (size_t) n * dout, 0) != OK)
         rc = ERR_ALLOC;
     if (rc == OK) rc = work_alloc(w, din, hid, dout, n);
     if (rc == OK) {
@@ -659,10 +659,10 @@ int guessnet_grad(int din, int hid, int dout, const float *params, const float *
         *loss = (float) l;
     }
     work_free(w);
-    cudaFree(dp);
-    cudaFree(dg);
-    cudaFree(dX);
-    cudaFree(dT);
+    dev_free(dp, 0);
+    dev_free(dg, 0);
+    dev_free(dX, 0);
+    dev_free(dT, 0);
     cudaStreamDestroy(s);
     return rc;
 }

@@ -1272,8 +1272,8 @@ struct KMixBatch {
 void kmix_batch_destroy(KMixBatch *b)
 {
     if (!b) return;
-    cudaFree(b->d_mols);
-    cudaFree(b->d_starts);
+    dev_free(b->d_mols, 0);
+    dev_free(b->d_starts, 0);
     delete b;
 }
 
@@ -1312,8 +1312,8 @@ int kmix_batch_create(KMixBatch **out, KMix *const *ks, int n, cudaStream_t s)
         b->max_bn = std::max(b->max_bn, d.bn);
     }
     b->h_starts.assign(2 * (n + 1), 0);
-    if (cudaMalloc(&b->d_mols, sizeof(KMixDev) * n) != cudaSuccess ||
-        cudaMalloc(&b->d_starts, sizeof(int) * 2 * (n + 1)) != cudaSuccess ||
+    if (dev_malloc((void **) &b->d_mols, sizeof(KMixDev) * n, s) != OK ||
+        dev_malloc((void **) &b->d_starts, sizeof(int) * 2 * (n + 1), s) != OK ||
         cudaMemcpyAsync(b->d_mols, h.data(), sizeof(KMixDev) * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) {
         cudaGetLastError();

@@ -390,10 +390,17 @@ void dfree(Engine *e, void *p)
     if (it != e->allocs.end()) e->allocs.erase(it);
 }
 
+// Copy to a host mirror, in order on the engine's stream (the caller waits for it: a pinned mirror is
+// written by the copy engine while the host goes on).
+void d2h_async(Engine *e, void *dst, const void *src, size_t bytes)
+{
+    cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->s);
+    e->d2h += (long long) bytes;
+}
 void d2h(Engine *e, void *dst, const void *src, size_t bytes)
 {
-    cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
-    e->d2h += (long long) bytes;
+    d2h_async(e, dst, src, bytes);
+    cudaStreamSynchronize(e->s);
 }
 
 template <typename T>
@@ -505,6 +512,86 @@ std::mutex &amaps_mu()
     return *mu;
 }
 
+// Page-locked host blocks. A process keeps at most PIN_MAX bytes of them,
+// live and idle together; what engines give back waits here for the next engine
+// of the same sizes, since locking and unlocking pages (and freeing any driver
+// allocation) goes through the kernel driver: 8 MB take 2 to 4 ms, and on a
+// machine whose driver is busy with other processes one cudaFreeHost was seen to
+// take 0.2 to 0.8 s of a job of 0.5 s. Idle blocks of other sizes make room.
+class PinPool {
+    static constexpr size_t PIN_MAX = (size_t) 256 << 20, PIN_ROUND = (size_t) 64 << 10;
+    static constexpr int SLOT = 256, SLOTS = 64;   // small blocks: slots of a slab that stays
+    std::mutex mu_;
+    std::map<void *, size_t> live_;
+    std::multimap<size_t, void *> idle_;
+    std::vector<void *> slots_;
+    size_t total_ = 0;
+
+public:
+    static PinPool &get()
+    {
+        static auto *p = new PinPool;   // outlives static destruction
+        return *p;
+    }
+    // nullptr: no room, or no page-locked memory to be had (the caller takes pageable memory)
+    void *take(size_t bytes)
+    {
+        const size_t len = (bytes + PIN_ROUND - 1) / PIN_ROUND * PIN_ROUND;
+        std::lock_guard<std::mutex> lk(mu_);
+        auto it = idle_.find(len);
+        void *b = nullptr;
+        if (it != idle_.end()) {
+            b = it->second;
+            idle_.erase(it);
+        } else {
+            while (total_ + len > PIN_MAX && !idle_.empty()) {
+                cudaFreeHost(idle_.begin()->second);
+                total_ -= idle_.begin()->first;
+                idle_.erase(idle_.begin());
+            }
+            if (total_ + len > PIN_MAX) return nullptr;
+            if (cudaHostAlloc(&b, len, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            total_ += len;
+        }
+        live_[b] = len;
+        return b;
+    }
+    bool give(void *b)   // false: not one of these
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        auto it = live_.find(b);
+        if (it == live_.end()) return false;
+        idle_.emplace(it->second, b);
+        live_.erase(it);
+        return true;
+    }
+    void *take_slot()
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (slots_.empty()) {
+            char *b = nullptr;
+            if (cudaHostAlloc((void **) &b, SLOT * SLOTS, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            for (int k = 0; k < SLOTS; k++) slots_.push_back(b + k * SLOT);
+        }
+        void *p = slots_.back();
+        slots_.pop_back();
+        return p;
+    }
+    void give_slot(void *p)
+    {
+        if (!p) return;
+        std::lock_guard<std::mutex> lk(mu_);
+        slots_.push_back(p);
+    }
+    static_assert(sizeof(RefineCtl) <= SLOT, "a slot holds the refinement's control block");
+};
+
 void *amalloc(size_t bytes)
 {
     if (bytes == 0) bytes = 64;
@@ -524,7 +611,7 @@ void *amalloc(size_t bytes)
 
 void afree(void *p)
 {
-    if (!p) return;
+    if (!p || PinPool::get().give(p)) return;
     size_t len = 0;
     {
         std::lock_guard<std::mutex> lk(amaps_mu());
@@ -536,6 +623,16 @@ void afree(void *p)
     }
     if (len) munmap(p, len);
     else free(p);
+}
+
+// A mirror that calls fill from the device again and again: page-locked from ABIG bytes on where the pool has
+// room, zeroed on the engine's stream (init waits for it); else as amalloc.
+void *amalloc_filled(Engine *e, size_t bytes)
+{
+    void *b = bytes >= ABIG ? PinPool::get().take(bytes) : nullptr;
+    if (!b) return amalloc(bytes);
+    fill((double *) b, 0.0, (bytes + 7) / 8, e->s);
+    return b;
 }
 
 #define RC(x)                    \
@@ -610,13 +707,9 @@ int init_impl(TinySCF_t t, const char *bas_fname, const char *df_bas_fname, cons
 
     // host mirrors
     size_t nn = (size_t) nbf * nbf;
-    t->sp_scrval = (double *) amalloc(sizeof(double) * t->nshellpairs);
-    t->bf_pair_scrval = (double *) amalloc(sizeof(double) * nn);
     t->df_sp_scrval = (double *) amalloc(sizeof(double) * t->df_nshells);
     t->uniq_sp_lid = (int *) amalloc(sizeof(int) * t->num_uniq_sp);
     t->uniq_sp_rid = (int *) amalloc(sizeof(int) * t->num_uniq_sp);
-    t->bf_pair_mask = (int *) amalloc(sizeof(int) * nn);
-    t->bf_pair_j = (int *) amalloc(sizeof(int) * nn);
     t->bf_pair_diag = (int *) amalloc(sizeof(int) * nbf);
     t->bf_mask_displs = (int *) amalloc(sizeof(int) * (nbf + 1));
     t->shell_bf_sind = (int *) amalloc(sizeof(int) * (t->nshells + 1));
@@ -627,9 +720,7 @@ int init_impl(TinySCF_t t, const char *bas_fname, const char *df_bas_fname, cons
     for (int i = 0; i < t->nshells; i++) t->shell_bf_num[i] = ncart(e->sh.am[i]);
     for (int i = 0; i <= t->df_nshells; i++) t->df_shell_bf_sind[i] = e->ash.bfoff[i];
     for (int i = 0; i < t->df_nshells; i++) t->df_shell_bf_num[i] = ncart(e->ash.am[i]);
-    double **mats[] = {&t->Hcore_mat, &t->S_mat, &t->F_mat, &t->D_mat, &t->J_mat, &t->K_mat, &t->X_mat, &t->tmp_mat};
-    for (double **m : mats) *m = (double *) amalloc(sizeof(double) * nn);
-    t->Cocc_mat = (double *) amalloc(sizeof(double) * nbf * t->n_occ);
+    t->tmp_mat = (double *) amalloc(sizeof(double) * nn);
     t->eigval = (double *) amalloc(sizeof(double) * nbf);
     t->ev_idx = (int *) amalloc(sizeof(int) * nbf);
     for (int i = 0; i < nbf; i++) t->ev_idx[i] = i;
@@ -653,6 +744,14 @@ int init_impl(TinySCF_t t, const char *bas_fname, const char *df_bas_fname, cons
         e->tsum[k] = 0.0;
         e->tcnt[k] = 0;
     }
+    // host mirrors that the device fills
+    double **mats[] = {&t->Hcore_mat, &t->S_mat, &t->F_mat, &t->D_mat, &t->J_mat, &t->K_mat, &t->X_mat,
+                       &t->bf_pair_scrval};
+    for (double **m : mats) *m = (double *) amalloc_filled(e, sizeof(double) * nn);
+    t->Cocc_mat = (double *) amalloc_filled(e, sizeof(double) * nbf * t->n_occ);
+    t->sp_scrval = (double *) amalloc_filled(e, sizeof(double) * t->nshellpairs);
+    t->bf_pair_mask = (int *) amalloc_filled(e, sizeof(int) * nn);
+    t->bf_pair_j = (int *) amalloc_filled(e, sizeof(int) * nn);
     boys_table_init(e->s);
     RC(upload_shells(e, e->sh, MAX_L_ORB, e->dsh));
     RC(upload_shells(e, e->ash, MAX_L_AUX, e->dash));
@@ -1229,19 +1328,38 @@ int fock_device(TinySCF_t t, bool force_fp64 = false)
     return cuda_rc("Fock build");
 }
 
+// A caller's matrix into its mirror and from there, page-locked, to the device (in order on the engine's
+// stream; the caller waits). The caller may pass the mirror itself.
+int h2d_mirror(Engine *e, double *dev, double *mirror, const double *src, size_t bytes)
+{
+    if (src != mirror) memcpy(mirror, src, bytes);
+    return cudaMemcpyAsync(dev, mirror, bytes, cudaMemcpyHostToDevice, e->s) == cudaSuccess ? OK : ERR_CUDA;
+}
+
+// The engine's page-locked words that copies land in.
+int need_slots(Engine *e)
+{
+    if (!e->h_rctl) e->h_rctl = (RefineCtl *) PinPool::get().take_slot();
+    if (!e->h_E) e->h_E = (double *) PinPool::get().take_slot();
+    return e->h_rctl && e->h_E ? OK : ERR_ALLOC;
+}
+
 int fock_impl(TinySCF_t t, bool to_host)
 {
     Engine *e = E_(t);
     if (!e || e->stage < 5) return ERR_STATE;
     RC(fock_device(t));
+    if (to_host) {
+        // the energy lands in a page-locked slot: an unpinned word would make the copy wait on the host
+        d2h_async(e, t->J_mat, e->J, sizeof(double) * e->nn);
+        d2h_async(e, t->K_mat, e->K, sizeof(double) * e->nn);
+        d2h_async(e, t->F_mat, e->F, sizeof(double) * e->nn);
+        RC(need_slots(e));
+        d2h_async(e, e->h_E, e->E, sizeof(double));
+    }
     RC(sync_rc(e, "Fock build"));
     tcollect(e);
-    if (to_host) {
-        d2h(e, t->J_mat, e->J, sizeof(double) * e->nn);
-        d2h(e, t->K_mat, e->K, sizeof(double) * e->nn);
-        d2h(e, t->F_mat, e->F, sizeof(double) * e->nn);
-        d2h(e, &t->HF_energy, e->E, sizeof(double));
-    }
+    if (to_host) t->HF_energy = *e->h_E;
     return OK;
 }
 
@@ -1312,13 +1430,13 @@ int density_impl(TinySCF_t t, bool to_host)
     Engine *e = E_(t);
     if (!e || e->stage < 1) return ERR_STATE;
     RC(density_device(t));
+    if (to_host) {
+        d2h_async(e, t->D_mat, e->D, sizeof(double) * e->nn);
+        d2h_async(e, t->Cocc_mat, e->Cocc, sizeof(double) * t->nbasfuncs * t->n_occ);
+        d2h_async(e, t->eigval, e->w, sizeof(double) * t->nbasfuncs);
+    }
     RC(sync_rc(e, "density"));
     tcollect(e);
-    if (to_host) {
-        d2h(e, t->D_mat, e->D, sizeof(double) * e->nn);
-        d2h(e, t->Cocc_mat, e->Cocc, sizeof(double) * t->nbasfuncs * t->n_occ);
-        d2h(e, t->eigval, e->w, sizeof(double) * t->nbasfuncs);
-    }
     return OK;
 }
 
@@ -1328,17 +1446,17 @@ int sync_host_impl(TinySCF_t t)
     if (!e) return ERR_STATE;
     RC(sync_rc(e, "sync"));
     const int nbf = t->nbasfuncs;
-    d2h(e, t->S_mat, e->S, sizeof(double) * e->nn);
-    d2h(e, t->Hcore_mat, e->H, sizeof(double) * e->nn);
-    d2h(e, t->X_mat, e->X, sizeof(double) * e->nn);
-    d2h(e, t->F_mat, e->F_is_orth ? e->Fp : e->F, sizeof(double) * e->nn);
-    d2h(e, t->D_mat, e->D, sizeof(double) * e->nn);
-    d2h(e, t->J_mat, e->J, sizeof(double) * e->nn);
-    d2h(e, t->K_mat, e->K, sizeof(double) * e->nn);
-    d2h(e, t->Cocc_mat, e->Cocc, sizeof(double) * nbf * t->n_occ);
-    d2h(e, t->eigval, e->w, sizeof(double) * nbf);
+    d2h_async(e, t->S_mat, e->S, sizeof(double) * e->nn);
+    d2h_async(e, t->Hcore_mat, e->H, sizeof(double) * e->nn);
+    d2h_async(e, t->X_mat, e->X, sizeof(double) * e->nn);
+    d2h_async(e, t->F_mat, e->F_is_orth ? e->Fp : e->F, sizeof(double) * e->nn);
+    d2h_async(e, t->D_mat, e->D, sizeof(double) * e->nn);
+    d2h_async(e, t->J_mat, e->J, sizeof(double) * e->nn);
+    d2h_async(e, t->K_mat, e->K, sizeof(double) * e->nn);
+    d2h_async(e, t->Cocc_mat, e->Cocc, sizeof(double) * nbf * t->n_occ);
+    d2h_async(e, t->eigval, e->w, sizeof(double) * nbf);
     DiisState st;
-    d2h(e, &st, e->diis, sizeof(st));
+    d2h(e, &st, e->diis, sizeof(st));   // and waits for the copies before it
     t->DIIS_len = st.len;
     t->DIIS_bmax_id = st.bmax_id;
     t->DIIS_bmax = st.bmax;
@@ -1365,11 +1483,8 @@ int graph_capture(TinySCF_t t)
     const int n = t->nbasfuncs, o = t->n_occ;
     graph_release(e);
     if (!e->s_body) TSCF_CUDA_CHECK(cudaStreamCreateWithFlags(&e->s_body, cudaStreamNonBlocking));
-    if (!e->h_rctl) {
-        TSCF_CUDA_CHECK(cudaMallocHost(&e->h_rctl, sizeof(RefineCtl)));
-        TSCF_CUDA_CHECK(cudaMallocHost(&e->h_E, sizeof(double)));
-        RC(dalloc(e, &e->rctl, 1));
-    }
+    RC(need_slots(e));
+    if (!e->rctl) RC(dalloc(e, &e->rctl, 1));
     const bool refine = e->dmode == TINYSCF_DENSITY_REFINE && o > 0 && o < n;
     if (refine) {
         RefineCtl c{};
@@ -1609,8 +1724,8 @@ void free_impl(TinySCF_t t)
         graph_release(e);
         if (e->s_body) cudaStreamDestroy(e->s_body);
         lap(1);
-        if (e->h_rctl) cudaFreeHost(e->h_rctl);
-        if (e->h_E) cudaFreeHost(e->h_E);
+        PinPool::get().give_slot(e->h_rctl);
+        PinPool::get().give_slot(e->h_E);
         lap(2);
         guessnet_free(e->gnet);
         lap(3);
@@ -1716,23 +1831,21 @@ int TinySCF_set_density(TinySCF_t t, const double *D, const double *Cocc)
 {
     if (!t || !t->dev) return TINYSCF_ERR_STATE;
     Engine *e = E_(t);
-    if (D && cudaMemcpy(e->D, D, sizeof(double) * e->nn, cudaMemcpyHostToDevice) != cudaSuccess) return TINYSCF_ERR_CUDA;
     if (D || Cocc) e->d_from_cocc = false;   // a caller's pair need not satisfy D = Cocc Cocc^T
-    if (Cocc && cudaMemcpy(e->Cocc, Cocc, sizeof(double) * t->nbasfuncs * t->n_occ, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (D && h2d_mirror(e, e->D, t->D_mat, D, sizeof(double) * e->nn) != OK) return TINYSCF_ERR_CUDA;
+    if (Cocc && h2d_mirror(e, e->Cocc, t->Cocc_mat, Cocc, sizeof(double) * t->nbasfuncs * t->n_occ) != OK)
         return TINYSCF_ERR_CUDA;
-    if (D) memcpy(t->D_mat, D, sizeof(double) * e->nn);
-    if (Cocc) memcpy(t->Cocc_mat, Cocc, sizeof(double) * t->nbasfuncs * t->n_occ);
-    return TINYSCF_OK;
+    return cudaStreamSynchronize(e->s) == cudaSuccess ? TINYSCF_OK : TINYSCF_ERR_CUDA;
 }
 
 int TinySCF_set_fock(TinySCF_t t, const double *F, int orthogonal)
 {
     if (!t || !t->dev || !F) return TINYSCF_ERR_STATE;
     Engine *e = E_(t);
-    if (cudaMemcpy(orthogonal ? e->Fp : e->F, F, sizeof(double) * e->nn, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (h2d_mirror(e, orthogonal ? e->Fp : e->F, t->F_mat, F, sizeof(double) * e->nn) != OK ||
+        cudaStreamSynchronize(e->s) != cudaSuccess)
         return TINYSCF_ERR_CUDA;
     e->F_is_orth = orthogonal != 0;
-    memcpy(t->F_mat, F, sizeof(double) * e->nn);
     return TINYSCF_OK;
 }
 
