@@ -159,18 +159,23 @@ __global__ void __launch_bounds__(256, 1) k_halftransform_dmma(const double *__r
 }
 
 // ---- K half-transform on the FP64 tensor cores, persistent and pipelined.
-// CTA b takes the items b, b + grid, ... (item = row i, 64 occupied columns
-// s0.., 256 aux columns p0.., with the occupied tiles of one (i, p0) adjacent
-// so the gathered DF rows are reused from L2). The CSR chunks of 16 partner
-// rows (the K steps) of its items form one stream that cp.async copies
-// KH_STAGES - 1 steps ahead of the DMMA tiles: the gathers of the next chunks,
-// the tile math and the write-out of a finished item overlap. Each step's row
-// indices are read one step earlier still, so no copy waits on an index load.
-// Tiles and fragment layout are those of half_tile_dmma.
+// CTA b takes the items b, b + grid, ... (item = row i, S occupied columns
+// s0.., PW aux columns p0.., with the occupied tiles of one (i, p0) adjacent so
+// the gathered DF rows are reused from L2). The CSR chunks of 16 partner rows
+// (the K steps) of its items form one stream that cp.async copies KH_STAGES - 1
+// steps ahead of the DMMA tiles: the gathers of the next chunks, the tile math
+// and the write-out of a finished item overlap. Each step's row indices are
+// read one step earlier still, so no copy waits on an index load; the
+// fragments of the next four k are read before the DMMAs of the current four.
+//
+// Bound by the FP64 tensor cores, so the tile's S is fitted to n_occ: WS x WP
+// warps of 8 NX x 32 outputs, S = 8 WS NX the multiple of 8, 16 or 24 that holds
+// n_occ (up to 168, more in several tiles). With a fixed S = 64 C20H42's 81
+// occupied orbitals were 128 columns of work (2.55 ms, now 1.82 ms), 13 waters'
+// 65 were 128 (0.83 ms, now 0.53 ms). Summation order: k ascending in
+// every output, as one chain of multiply-adds (what DMMA does, bit for bit).
 constexpr int KH_STAGES = 4;
-constexpr int KH_AS = KH_S + 4, KH_BS = KH_P + 4;
-constexpr int KH_STAGE_DOUBLES = KT_K * (KH_AS + KH_BS);
-constexpr size_t KH_PIPE_SMEM = sizeof(double) * KH_STAGES * KH_STAGE_DOUBLES;
+constexpr int KH_SMAX = 168;
 
 __device__ __forceinline__ void cp_async8(double *dst, const double *src, int bytes)
 {
@@ -189,6 +194,15 @@ struct KhCursor {
     int item, i, s0, p0, r0, r_end, step, nsteps;
 };
 
+template <int WS, int NX, int WP>
+struct KhTile {
+    static constexpr int S = WS * NX * 8, P = WP * 32, THREADS = WS * WP * 32;
+    static constexpr int AS = S + 4, BS = P + 4;   // strides = 4 or 12 (mod 16) doubles: conflict-free fragments
+    static constexpr int STAGE = KT_K * (AS + BS);
+    static constexpr size_t SMEM = sizeof(double) * KH_STAGES * STAGE;
+};
+
+template <int S, int P>
 __device__ __forceinline__ void kh_set(KhCursor &c, int item, int n_items, int stiles, int ptiles,
                                        const int *__restrict__ displs)
 {
@@ -197,67 +211,80 @@ __device__ __forceinline__ void kh_set(KhCursor &c, int item, int n_items, int s
     const int per_row = stiles * ptiles;
     c.i = item / per_row;
     const int rem = item - c.i * per_row;
-    c.p0 = (rem / stiles) * KH_P;
-    c.s0 = (rem % stiles) * KH_S;
+    c.p0 = (rem / stiles) * P;
+    c.s0 = (rem % stiles) * S;
     c.r0 = displs[c.i];
     c.r_end = displs[c.i + 1];
     c.step = 0;
     c.nsteps = max(1, (c.r_end - c.r0 + KT_K - 1) / KT_K);   // a row without partners still writes its zeros
 }
 
+template <int S, int P>
 __device__ __forceinline__ void kh_next(KhCursor &c, int n_items, int stiles, int ptiles,
                                         const int *__restrict__ displs)
 {
     if (c.item >= n_items) return;
     if (++c.step < c.nsteps) c.r0 += KT_K;
-    else kh_set(c, c.item + gridDim.x, n_items, stiles, ptiles, displs);
+    else kh_set<S, P>(c, c.item + gridDim.x, n_items, stiles, ptiles, displs);
 }
 
-// VEC: 16-byte copies of the DF rows (naux even, so every row starts 16-byte aligned)
-template <bool VEC>
-__global__ void __launch_bounds__(256, 1)
+// VEC: 16-byte copies of the DF rows and stores of T (naux even, so every row starts 16-byte aligned)
+template <int WS, int NX, int WP, bool VEC>
+__global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
     k_halftransform_pipe(const double *__restrict__ B, const double *__restrict__ C, const int *__restrict__ csr_j,
                          const int *__restrict__ csr_u, const int *__restrict__ displs, int nocc, int naux,
                          double *__restrict__ T, int n_items, int stiles, int ptiles, unsigned long long *rowmax)
 {
+    using K = KhTile<WS, NX, WP>;
+    constexpr int S = K::S, PW = K::P, NT = K::THREADS;
     extern __shared__ __align__(16) double khsm[];
-    constexpr int NBR = VEC ? 8 : 16;   // DF rows whose copies this thread issues per step
+    constexpr int BCOPY = VEC ? 2 : 1;                      // doubles per B copy
+    constexpr int NBC = KT_K * PW / BCOPY, NB = (NBC + NT - 1) / NT;   // B copies per step, per thread
+    constexpr int NAC = KT_K * S, NA = (NAC + NT - 1) / NT;            // Cocc copies per step, per thread
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ws = (warp >> 2) * 32, wp = (warp & 3) * 64;
+    const int ws = (warp / WP) * NX * 8, wp = (warp % WP) * 32;
     const int fr = lane >> 2, fc = lane & 3;
-    int iu[NBR], ij[4];
+    int iu[NB], ij[NA];
     KhCursor P, Q;   // P: the next step to copy; Q: the step the tiles consume
-    kh_set(P, blockIdx.x, n_items, stiles, ptiles, displs);
+    kh_set<S, PW>(P, blockIdx.x, n_items, stiles, ptiles, displs);
     Q = P;
     auto load_idx = [&]() {   // row indices of P's step (-1: past the row, zero fill)
 #pragma unroll
-        for (int q = 0; q < NBR; q++) {
-            const int r = P.r0 + (VEC ? 2 * q + (tid >> 7) : q);
-            iu[q] = (P.item < n_items && r < P.r_end) ? csr_u[r] : -1;
+        for (int q = 0; q < NB; q++) {
+            const int c = tid + NT * q;
+            const int r = P.r0 + c / (PW / BCOPY);
+            iu[q] = (c < NBC && P.item < n_items && r < P.r_end) ? csr_u[r] : -1;
         }
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int r = P.r0 + 4 * q + (tid >> 6);
-            ij[q] = (P.item < n_items && r < P.r_end) ? csr_j[r] : -1;
+        for (int q = 0; q < NA; q++) {
+            const int c = tid + NT * q;
+            const int r = P.r0 + c / S;
+            ij[q] = (c < NAC && P.item < n_items && r < P.r_end) ? csr_j[r] : -1;
         }
     };
     auto issue = [&](int buf) {   // copies of P's step into stage buffer buf, one commit group
-        double *As = khsm + (size_t) buf * KH_STAGE_DOUBLES, *Bs = As + KT_K * KH_AS;
+        double *As = khsm + (size_t) buf * K::STAGE, *Bs = As + KT_K * K::AS;
         if (P.item < n_items) {
 #pragma unroll
-            for (int q = 0; q < NBR; q++) {
-                const int kk = VEC ? 2 * q + (tid >> 7) : q, cc = VEC ? (tid & 127) * 2 : tid;
-                const int pg = P.p0 + cc;
-                const bool ok = iu[q] >= 0 && pg < naux;
-                const double *src = ok ? B + (size_t) iu[q] * naux + pg : B;
-                if (VEC) cp_async16(&Bs[kk * KH_BS + cc], src, ok ? 16 : 0);
-                else cp_async8(&Bs[kk * KH_BS + cc], src, ok ? 8 : 0);
+            for (int q = 0; q < NB; q++) {
+                const int c = tid + NT * q;
+                if (NBC % NT == 0 || c < NBC) {
+                    const int kk = c / (PW / BCOPY), cc = (c % (PW / BCOPY)) * BCOPY;
+                    const int pg = P.p0 + cc;
+                    const bool ok = iu[q] >= 0 && pg < naux;
+                    const double *src = ok ? B + (size_t) iu[q] * naux + pg : B;
+                    if (VEC) cp_async16(&Bs[kk * K::BS + cc], src, ok ? 16 : 0);
+                    else cp_async8(&Bs[kk * K::BS + cc], src, ok ? 8 : 0);
+                }
             }
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int kk = 4 * q + (tid >> 6), cc = tid & 63, sg = P.s0 + cc;
-                const bool ok = ij[q] >= 0 && sg < nocc;
-                cp_async8(&As[kk * KH_AS + cc], ok ? C + (size_t) ij[q] * nocc + sg : C, ok ? 8 : 0);
+            for (int q = 0; q < NA; q++) {
+                const int c = tid + NT * q;
+                if (NAC % NT == 0 || c < NAC) {
+                    const int kk = c / S, cc = c % S, sg = P.s0 + cc;
+                    const bool ok = ij[q] >= 0 && sg < nocc;
+                    cp_async8(&As[kk * K::AS + cc], ok ? C + (size_t) ij[q] * nocc + sg : C, ok ? 8 : 0);
+                }
             }
         }
         cp_async_commit();
@@ -265,44 +292,57 @@ __global__ void __launch_bounds__(256, 1)
     for (int st = 0; st < KH_STAGES - 1; st++) {
         load_idx();
         issue(st);
-        kh_next(P, n_items, stiles, ptiles, displs);
+        kh_next<S, PW>(P, n_items, stiles, ptiles, displs);
     }
     load_idx();
-    double acc[4][8][2];
+    double acc[NX][4][2];
 #pragma unroll
-    for (int x = 0; x < 4; x++)
+    for (int x = 0; x < NX; x++)
 #pragma unroll
-        for (int y = 0; y < 8; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
+        for (int y = 0; y < 4; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
     for (int g = 0; Q.item < n_items; g++) {
         cp_async_wait<KH_STAGES - 2>();   // this thread's copies of step g have landed
         __syncthreads();                  // everyone's have, and step g - 1's buffer is free
-        issue((g + KH_STAGES - 1) % KH_STAGES);
-        kh_next(P, n_items, stiles, ptiles, displs);
-        load_idx();
-        const double *As = khsm + (size_t) (g % KH_STAGES) * KH_STAGE_DOUBLES, *Bs = As + KT_K * KH_AS;
+        const double *As = khsm + (size_t) (g % KH_STAGES) * K::STAGE + fc * K::AS + ws + fr;
+        const double *Bs = khsm + (size_t) (g % KH_STAGES) * K::STAGE + KT_K * K::AS + fc * K::BS + wp + fr;
+        double a[2][NX], b[2][4];
+        auto frag = [&](int w, int k4) {
+#pragma unroll
+            for (int x = 0; x < NX; x++) a[w][x] = As[k4 * K::AS + 8 * x];
+#pragma unroll
+            for (int y = 0; y < 4; y++) b[w][y] = Bs[k4 * K::BS + 8 * y];
+        };
+        frag(0, 0);
 #pragma unroll
         for (int k4 = 0; k4 < KT_K; k4 += 4) {
-            double a[4], b[8];
+            const int w = (k4 / 4) & 1;
+            if (k4 + 4 < KT_K) frag(w ^ 1, k4 + 4);
 #pragma unroll
-            for (int x = 0; x < 4; x++) a[x] = As[(k4 + fc) * KH_AS + ws + 8 * x + fr];
+            for (int x = 0; x < NX; x++)
 #pragma unroll
-            for (int y = 0; y < 8; y++) b[y] = Bs[(k4 + fc) * KH_BS + wp + 8 * y + fr];
-#pragma unroll
-            for (int x = 0; x < 4; x++)
-#pragma unroll
-                for (int y = 0; y < 8; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], a[x], b[y]);
+                for (int y = 0; y < 4; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], a[w][x], b[w][y]);
+            if (k4 == 0) {   // the next copies go out behind the first DMMAs
+                issue((g + KH_STAGES - 1) % KH_STAGES);
+                kh_next<S, PW>(P, n_items, stiles, ptiles, displs);
+                load_idx();
+            }
         }
         if (++Q.step == Q.nsteps) {   // item done: write its tile, start the next
             double amax = 0.0;        // max |T| of the tile (padding entries are zero)
 #pragma unroll
-            for (int x = 0; x < 4; x++) {
+            for (int x = 0; x < NX; x++) {
                 const int sg = Q.s0 + ws + 8 * x + fr;
                 double *row = T + ((size_t) Q.i * nocc + (sg < nocc ? sg : 0)) * naux;
 #pragma unroll
-                for (int y = 0; y < 8; y++) {
+                for (int y = 0; y < 4; y++) {
                     const int pg = Q.p0 + wp + 8 * y + 2 * fc;
-                    if (sg < nocc && pg < naux) row[pg] = acc[x][y][0];
-                    if (sg < nocc && pg + 1 < naux) row[pg + 1] = acc[x][y][1];
+                    if (VEC) {
+                        if (sg < nocc && pg < naux)
+                            *reinterpret_cast<double2 *>(row + pg) = make_double2(acc[x][y][0], acc[x][y][1]);
+                    } else {
+                        if (sg < nocc && pg < naux) row[pg] = acc[x][y][0];
+                        if (sg < nocc && pg + 1 < naux) row[pg + 1] = acc[x][y][1];
+                    }
                     amax = fmax(amax, fmax(fabs(acc[x][y][0]), fabs(acc[x][y][1])));
                     acc[x][y][0] = acc[x][y][1] = 0.0;
                 }
@@ -311,154 +351,61 @@ __global__ void __launch_bounds__(256, 1)
                 for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffff, amax, o));
                 if (lane == 0 && amax > 0.0) atomicMax(rowmax + Q.i, (unsigned long long) __double_as_longlong(amax));
             }
-            kh_set(Q, Q.item + gridDim.x, n_items, stiles, ptiles, displs);
+            kh_set<S, PW>(Q, Q.item + gridDim.x, n_items, stiles, ptiles, displs);
         }
     }
     cp_async_wait<0>();
 }
 
-// ---- the same half-transform with 168 x 128 tiles over 12 warps (3 x 4 warps
-// of 56 x 32): n_occ up to 168 in one tile, so each CSR chunk of B is gathered
-// once per (row, aux tile) instead of once per 64-wide occupied tile, and
-// n_occ = 161 pads to 168 instead of 192.
-constexpr int KH2_S = 168, KH2_P = 128, KH2_THREADS = 384;
-constexpr int KH2_AS = KH2_S + 4, KH2_BS = KH2_P + 4;   // strides = 12 / 4 (mod 16) doubles: conflict-free fragments
-constexpr int KH2_STAGE_DOUBLES = KT_K * (KH2_AS + KH2_BS);
-constexpr size_t KH2_PIPE_SMEM = sizeof(double) * KH_STAGES * KH2_STAGE_DOUBLES;
-constexpr int KH2_NA = KT_K * KH2_S / KH2_THREADS;   // 7 Cocc copies per thread per step
-
-__device__ __forceinline__ void kh2_set(KhCursor &c, int item, int n_items, int stiles, int ptiles,
-                                        const int *__restrict__ displs)
+template <int WS, int NX, int WP>
+static void launch_half_pipe(const FockPlan &p, const double *C, double *T, unsigned long long *rowmax, cudaStream_t s)
 {
-    c.item = item;
-    if (item >= n_items) return;
-    const int per_row = stiles * ptiles;
-    c.i = item / per_row;
-    const int rem = item - c.i * per_row;
-    c.p0 = (rem / stiles) * KH2_P;
-    c.s0 = (rem % stiles) * KH2_S;
-    c.r0 = displs[c.i];
-    c.r_end = displs[c.i + 1];
-    c.step = 0;
-    c.nsteps = max(1, (c.r_end - c.r0 + KT_K - 1) / KT_K);
+    using K = KhTile<WS, NX, WP>;
+    const int stiles = (p.nocc + K::S - 1) / K::S, ptiles = (p.naux + K::P - 1) / K::P;
+    const long long items = (long long) p.nbf * stiles * ptiles;
+    auto go = [&](auto kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) K::SMEM);
+        int per = 1;   // the small tiles fit several times on an SM
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, K::THREADS, K::SMEM);
+        const int grid = (int) std::min<long long>(items, (long long) num_sms() * std::max(per, 1));
+        kernel<<<grid, K::THREADS, K::SMEM, s>>>(p.B, C, p.csr_j, p.csr_u, p.csr_displs, p.nocc, p.naux, T, (int) items,
+                                                 stiles, ptiles, rowmax);
+    };
+    if (p.naux % 2 == 0) go(k_halftransform_pipe<WS, NX, WP, true>);
+    else go(k_halftransform_pipe<WS, NX, WP, false>);
 }
 
-__device__ __forceinline__ void kh2_next(KhCursor &c, int n_items, int stiles, int ptiles,
-                                         const int *__restrict__ displs)
+// The tile for n_occ: one row of warps up to 56 occupied orbitals, two up to
+// 112, three up to 168 and for the equal parts of more; wide: 256 or 192 aux
+// columns for the first two (fewer re-reads of Cocc), narrow: 128 (less padding
+// of a short aux dimension); the autotuner times both.
+static void half_pipe(const FockPlan &p, const double *C, double *T, unsigned long long *rowmax, cudaStream_t s, bool wide)
 {
-    if (c.item >= n_items) return;
-    if (++c.step < c.nsteps) c.r0 += KT_K;
-    else kh2_set(c, c.item + gridDim.x, n_items, stiles, ptiles, displs);
-}
-
-template <bool VEC>
-__global__ void __launch_bounds__(KH2_THREADS, 1)
-    k_halftransform_pipe2(const double *__restrict__ B, const double *__restrict__ C, const int *__restrict__ csr_j,
-                          const int *__restrict__ csr_u, const int *__restrict__ displs, int nocc, int naux,
-                          double *__restrict__ T, int n_items, int stiles, int ptiles, unsigned long long *rowmax)
-{
-    extern __shared__ __align__(16) double khsm[];
-    constexpr int BCOPY = VEC ? 2 : 1;                                   // doubles per B copy
-    constexpr int NBC = KT_K * KH2_P / BCOPY;                            // B copies per step
-    constexpr int NB = (NBC + KH2_THREADS - 1) / KH2_THREADS;            // per thread
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ws = (warp >> 2) * 56, wp = (warp & 3) * 32;
-    const int fr = lane >> 2, fc = lane & 3;
-    int iu[NB], ij[KH2_NA];
-    KhCursor P, Q;
-    kh2_set(P, blockIdx.x, n_items, stiles, ptiles, displs);
-    Q = P;
-    auto load_idx = [&]() {
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-            const int c = tid + KH2_THREADS * q;
-            const int r = P.r0 + c / (KH2_P / BCOPY);
-            iu[q] = (c < NBC && P.item < n_items && r < P.r_end) ? csr_u[r] : -1;
-        }
-#pragma unroll
-        for (int q = 0; q < KH2_NA; q++) {
-            const int r = P.r0 + (tid + KH2_THREADS * q) / KH2_S;
-            ij[q] = (P.item < n_items && r < P.r_end) ? csr_j[r] : -1;
-        }
-    };
-    auto issue = [&](int buf) {
-        double *As = khsm + (size_t) buf * KH2_STAGE_DOUBLES, *Bs = As + KT_K * KH2_AS;
-        if (P.item < n_items) {
-#pragma unroll
-            for (int q = 0; q < NB; q++) {
-                const int c = tid + KH2_THREADS * q;
-                if (c < NBC) {
-                    const int kk = c / (KH2_P / BCOPY), cc = (c % (KH2_P / BCOPY)) * BCOPY;
-                    const int pg = P.p0 + cc;
-                    const bool ok = iu[q] >= 0 && pg < naux;
-                    const double *src = ok ? B + (size_t) iu[q] * naux + pg : B;
-                    if (VEC) cp_async16(&Bs[kk * KH2_BS + cc], src, ok ? 16 : 0);
-                    else cp_async8(&Bs[kk * KH2_BS + cc], src, ok ? 8 : 0);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < KH2_NA; q++) {
-                const int c = tid + KH2_THREADS * q;
-                const int kk = c / KH2_S, cc = c % KH2_S, sg = P.s0 + cc;
-                const bool ok = ij[q] >= 0 && sg < nocc;
-                cp_async8(&As[kk * KH2_AS + cc], ok ? C + (size_t) ij[q] * nocc + sg : C, ok ? 8 : 0);
-            }
-        }
-        cp_async_commit();
-    };
-    for (int st = 0; st < KH_STAGES - 1; st++) {
-        load_idx();
-        issue(st);
-        kh2_next(P, n_items, stiles, ptiles, displs);
+    const int tiles = (p.nocc + KH_SMAX - 1) / KH_SMAX, o = (p.nocc + tiles - 1) / tiles;
+    const int ws = o <= 56 ? 1 : (o <= 112 ? 2 : 3), nx = (o + 8 * ws - 1) / (8 * ws);
+#define TSCF_HALF(WS, NX, WIDE)                                          \
+    case 10 * WS + NX:                                                   \
+        if (wide) launch_half_pipe<WS, NX, WIDE>(p, C, T, rowmax, s);    \
+        else launch_half_pipe<WS, NX, 4>(p, C, T, rowmax, s);            \
+        break;
+    switch (10 * ws + nx) {
+        TSCF_HALF(1, 1, 8)
+        TSCF_HALF(1, 2, 8)
+        TSCF_HALF(1, 3, 8)
+        TSCF_HALF(1, 4, 8)
+        TSCF_HALF(1, 5, 8)
+        TSCF_HALF(1, 6, 8)
+        TSCF_HALF(1, 7, 8)
+        TSCF_HALF(2, 4, 6)
+        TSCF_HALF(2, 5, 6)
+        TSCF_HALF(2, 6, 6)
+        TSCF_HALF(2, 7, 6)
+        TSCF_HALF(3, 5, 4)
+        TSCF_HALF(3, 6, 4)
+        TSCF_HALF(3, 7, 4)
+    default: break;   // none left: a part of n_occ in 1..56, 57..112 or 113..168 has these NX
     }
-    load_idx();
-    double acc[7][4][2];
-#pragma unroll
-    for (int x = 0; x < 7; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
-    for (int g = 0; Q.item < n_items; g++) {
-        cp_async_wait<KH_STAGES - 2>();
-        __syncthreads();
-        issue((g + KH_STAGES - 1) % KH_STAGES);
-        kh2_next(P, n_items, stiles, ptiles, displs);
-        load_idx();
-        const double *As = khsm + (size_t) (g % KH_STAGES) * KH2_STAGE_DOUBLES, *Bs = As + KT_K * KH2_AS;
-#pragma unroll
-        for (int k4 = 0; k4 < KT_K; k4 += 4) {
-            double a[7], b[4];
-#pragma unroll
-            for (int x = 0; x < 7; x++) a[x] = As[(k4 + fc) * KH2_AS + ws + 8 * x + fr];
-#pragma unroll
-            for (int y = 0; y < 4; y++) b[y] = Bs[(k4 + fc) * KH2_BS + wp + 8 * y + fr];
-#pragma unroll
-            for (int x = 0; x < 7; x++)
-#pragma unroll
-                for (int y = 0; y < 4; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], a[x], b[y]);
-        }
-        if (++Q.step == Q.nsteps) {
-            double amax = 0.0;
-#pragma unroll
-            for (int x = 0; x < 7; x++) {
-                const int sg = Q.s0 + ws + 8 * x + fr;
-                double *row = T + ((size_t) Q.i * nocc + (sg < nocc ? sg : 0)) * naux;
-#pragma unroll
-                for (int y = 0; y < 4; y++) {
-                    const int pg = Q.p0 + wp + 8 * y + 2 * fc;
-                    if (sg < nocc && pg < naux) row[pg] = acc[x][y][0];
-                    if (sg < nocc && pg + 1 < naux) row[pg + 1] = acc[x][y][1];
-                    amax = fmax(amax, fmax(fabs(acc[x][y][0]), fabs(acc[x][y][1])));
-                    acc[x][y][0] = acc[x][y][1] = 0.0;
-                }
-            }
-            if (rowmax) {
-                for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffff, amax, o));
-                if (lane == 0 && amax > 0.0) atomicMax(rowmax + Q.i, (unsigned long long) __double_as_longlong(amax));
-            }
-            kh2_set(Q, Q.item + gridDim.x, n_items, stiles, ptiles, displs);
-        }
-    }
-    cp_async_wait<0>();
+#undef TSCF_HALF
 }
 
 // K partial tiles: upper tile pairs (bi <= bj) of 64x64, split over the
@@ -513,39 +460,9 @@ void build_K_halftransform(const FockPlan &p, const double *d_Cocc, double *d_T,
 {
     if (p.nbf <= 0 || p.nocc <= 0 || p.naux <= 0) return;   // T is empty: no grid to launch
     g_launches++;
-    if (wide == 4) {
+    if (wide >= 3) {
         if (d_rowmax) cudaMemsetAsync(d_rowmax, 0, sizeof(unsigned long long) * p.nbf, s);
-        const int stiles = (p.nocc + KH2_S - 1) / KH2_S, ptiles = (p.naux + KH2_P - 1) / KH2_P;
-        const long long items = (long long) p.nbf * stiles * ptiles;
-        cudaFuncSetAttribute(k_halftransform_pipe2<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int) KH2_PIPE_SMEM);
-        cudaFuncSetAttribute(k_halftransform_pipe2<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int) KH2_PIPE_SMEM);
-        const int grid = (int) std::min<long long>(items, num_sms());
-        if (p.naux % 2 == 0)
-            k_halftransform_pipe2<true><<<grid, KH2_THREADS, KH2_PIPE_SMEM, s>>>(
-                p.B, d_Cocc, p.csr_j, p.csr_u, p.csr_displs, p.nocc, p.naux, d_T, (int) items, stiles, ptiles, d_rowmax);
-        else
-            k_halftransform_pipe2<false><<<grid, KH2_THREADS, KH2_PIPE_SMEM, s>>>(
-                p.B, d_Cocc, p.csr_j, p.csr_u, p.csr_displs, p.nocc, p.naux, d_T, (int) items, stiles, ptiles, d_rowmax);
-    } else if (wide == 3) {
-        if (d_rowmax) cudaMemsetAsync(d_rowmax, 0, sizeof(unsigned long long) * p.nbf, s);
-        const int stiles = (p.nocc + KH_S - 1) / KH_S, ptiles = (p.naux + KH_P - 1) / KH_P;
-        const long long items = (long long) p.nbf * stiles * ptiles;
-        const int sms = num_sms();
-        cudaFuncSetAttribute(k_halftransform_pipe<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int) KH_PIPE_SMEM);
-        cudaFuncSetAttribute(k_halftransform_pipe<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int) KH_PIPE_SMEM);
-        const int grid = (int) std::min<long long>(items, sms);
-        if (p.naux % 2 == 0)
-            k_halftransform_pipe<true><<<grid, 256, KH_PIPE_SMEM, s>>>(p.B, d_Cocc, p.csr_j, p.csr_u, p.csr_displs,
-                                                                       p.nocc, p.naux, d_T, (int) items, stiles,
-                                                                       ptiles, d_rowmax);
-        else
-            k_halftransform_pipe<false><<<grid, 256, KH_PIPE_SMEM, s>>>(p.B, d_Cocc, p.csr_j, p.csr_u,
-                                                                        p.csr_displs, p.nocc, p.naux, d_T,
-                                                                        (int) items, stiles, ptiles, d_rowmax);
+        half_pipe(p, d_Cocc, d_T, d_rowmax, s, wide == 4);
     } else if (wide) {
         dim3 g1((p.naux + KH_P - 1) / KH_P, (p.nocc + KH_S - 1) / KH_S, p.nbf);
         if (wide == 2)

@@ -202,10 +202,9 @@ void build_J_f32(const FockPlan &p, const float *B32, const double *d_D, double 
 void convert_f32(const double *in, float *out, size_t n, cudaStream_t s);
 // K from Cocc (build_Fock.c:244-347): T(i,s,P) = sum_j C(j,s) B(ij,P) ...
 // wide = 1: 64 x 256 FFMA tiles (k_halftransform_wide), 2: 64 x 256 DMMA tiles
-// (k_halftransform_dmma), 3: the same DMMA tiles in persistent CTAs with a
-// cp.async pipeline over the CSR chunks (k_halftransform_pipe), 4: 168 x 128
-// DMMA tiles over 12 warps in the same pipeline (k_halftransform_pipe2), 0:
-// 64 x 64 FFMA tiles
+// (k_halftransform_dmma), 3 and 4: DMMA tiles fitted to n_occ in persistent CTAs
+// with a cp.async pipeline over the CSR chunks (k_halftransform_pipe), narrow and
+// wide in the aux dimension, 0: 64 x 64 FFMA tiles
 // d_rowmax (wide = 3 or 4, else ignored): max_q |T(i, q)| of every row as
 // double bits, for the integer-tensor-core K.
 void build_K_halftransform(const FockPlan &p, const double *d_Cocc, double *d_T, cudaStream_t s, int wide = 0,
