@@ -1,7 +1,8 @@
 """The exchange half-transform's tiles fitted to the occupied dimension: at the
-edges of each warp layout (one, two or three rows of warps) and of its blocks of
-8, 16 and 24 occupied orbitals, with an even and an odd number of auxiliary
-functions, both aux widths, against the 64 x 64 tile kernel on the same density.
+edges of each warp layout (one, two or three rows of warps, more than one tile)
+and of its blocks of 8, 16 and 24 occupied orbitals, both aux widths, against the
+64 x 64 tile kernel on the same density. (An odd number of auxiliary functions
+takes the copies of k_halftransform_pipe: test_gpu_tune.py's HCN.)
 
 Every output is one chain of multiply-adds over the same k in all of these
 kernels, so T is the same bit for bit; K = T T^T then runs on the same kernel
@@ -38,8 +39,8 @@ def atoms(name):
     return geometry.alkane(n) if kind == "c" else geometry.water_cluster(11, n, n)
 
 
-# o = 5, 17, 25, 55, 57 (c14), 65 (w13), 81 (c20), 113 (c28)
-@pytest.mark.parametrize("name", ["w1", "c4", "c6", "w11", "c14", "w13", "c20", "c28"])
+# o = 5, 17, 55, 57 (c14), 65 (w13), 85 (c21), 89 (c22), 125 (c31), 129 (c32), 169 (c42: two parts of 85)
+@pytest.mark.parametrize("name", ["w1", "c4", "w11", "c14", "w13", "c21", "c22", "c31", "c32", "c42"])
 def test_fitted_tiles_equal_square_tiles(tmp_path, name):
     xyz = str(tmp_path / "m.xyz")
     geometry.write_xyz(xyz, atoms(name))

@@ -1106,10 +1106,12 @@ __device__ __forceinline__ void secular_parts(const double *sd, const double *sz
             d += q * q;
         }
     }
-    p1 = rho * warp_sum_bcast(a);
-    dp1 = rho * warp_sum_bcast(b);
-    p2 = rho * warp_sum_bcast(c);
-    dp2 = rho * warp_sum_bcast(d);
+    double v[4] = {a, b, c, d};   // the sums of four shuffle trees, in 6 shuffles instead of 20
+    const double x = warp_sums<4>(v, lane);
+    p1 = rho * __shfl_sync(0xffffffffu, x, trc_lane<4>(0));
+    dp1 = rho * __shfl_sync(0xffffffffu, x, trc_lane<4>(1));
+    p2 = rho * __shfl_sync(0xffffffffu, x, trc_lane<4>(2));
+    dp2 = rho * __shfl_sync(0xffffffffu, x, trc_lane<4>(3));
 }
 
 // Roots of f(l) = 1 + rho sum_i z_i^2 / (d_i - l) = 0, one warp per root:
@@ -1120,8 +1122,14 @@ __device__ __forceinline__ void secular_parts(const double *sd, const double *sz
 // poles around the root) and takes the model's root inside the bracket;
 // a bisection step (geometric while the bracket spans more than a factor 4)
 // when it falls outside. Stops when the step is below 2 eps |tau| or the
-// bracket closes.
-__global__ void __launch_bounds__(256) k_dc_secular(DcNodes nd, DcPos ps, const int2 *tab)
+// bracket closes. At the root the model's step is rounding and often falls on the
+// bracket's end, so most roots go through tens of bisections of a wide bracket
+// before it closes (50 us per level however few roots). at_noise stops where
+// |f| is within the rounding of its own terms instead, which determines the root
+// as far as f can (the criterion of LAPACK's dlaed4): 13 us. The bracketed
+// stop stays for the eigenbases of the accelerated form and of X and (P|Q)^-1/2,
+// whose users amplify the last bits (1e-16 in X moves its density by 1e-9).
+__global__ void __launch_bounds__(256) k_dc_secular(DcNodes nd, DcPos ps, const int2 *tab, bool at_noise)
 {
     extern __shared__ double dsm[];
     const int2 tb = tab[blockIdx.x];
@@ -1173,6 +1181,7 @@ __global__ void __launch_bounds__(256) k_dc_secular(DcNodes nd, DcPos ps, const 
             secular_parts(sd, sz, k, j, rho, dorg, tau, lane, p1, dp1, p2, dp2);
             const double f = 1.0 + p1 + p2;
             if (f == 0.0) break;
+            if (at_noise && fabs(f) <= DBL_EPSILON * (8.0 * (1.0 + fabs(p1) + fabs(p2)) + fabs(tau) * (dp1 + dp2))) break;
             if (f < 0.0) a = tau; else b = tau;
             if (!(b - a > 4.0 * DBL_EPSILON * fmax(fabs(a), fabs(b)))) break;
             // two-pole model: C + s1 / (del1 - x) + s2 / (del2 - x) = 0
@@ -1709,7 +1718,7 @@ int tridiagonalize(Eig *E, const double *d_A, cudaStream_t s)
 }
 
 // Eigenvectors of T into the columns of the returned buffer (E->A or E->Qb).
-int divide_conquer(Eig *E, cudaStream_t s, double **out)
+int divide_conquer(Eig *E, cudaStream_t s, double **out, bool at_noise)
 {
     const int n = E->n;
     const size_t nn = (size_t) n * n;
@@ -1725,7 +1734,7 @@ int divide_conquer(Eig *E, cudaStream_t s, double **out)
         const double *Qin = buf[(L.depth + 1) % 2];
         double *Qout = buf[L.depth % 2];
         k_dc_deflate<<<L.nnodes, 512, 20 * m, s>>>(E->nodes, E->pos, Qin, E->e, n, L.node0);
-        k_dc_secular<<<L.nw, 256, 16 * m, s>>>(E->nodes, E->pos, E->tab_w + L.w0);
+        k_dc_secular<<<L.nw, 256, 16 * m, s>>>(E->nodes, E->pos, E->tab_w + L.w0, at_noise);
         k_dc_zhat<<<L.nw, 256, 24 * m, s>>>(E->nodes, E->pos, E->tab_w + L.w0);
         k_dc_norms<<<L.nw, 256, 16 * m, s>>>(E->nodes, E->pos, E->tab_w + L.w0);
         k_dc_order<<<L.nc, DC_CHUNK, 8 * m, s>>>(E->nodes, E->pos, E->tab_c + L.c0);
@@ -1767,7 +1776,7 @@ int back_transform(Eig *E, const double *Zc, double *d_V, cudaStream_t s)
 
 // Eigenvalues ascending into d_w, eigenvectors as rows of d_V (V[k*n + i] =
 // entry i of eigenvector k). d_V may alias d_A.
-int eig_run(Eig *E, const double *d_A, double *d_w, double *d_V, cudaStream_t s)
+int eig_run(Eig *E, const double *d_A, double *d_w, double *d_V, cudaStream_t s, bool at_noise)
 {
     if (!E) return ERR_STATE;
     const int n = E->n;
@@ -1779,7 +1788,7 @@ int eig_run(Eig *E, const double *d_A, double *d_w, double *d_V, cudaStream_t s)
     }
     RC_(tridiagonalize(E, d_A, s));
     double *Z = nullptr;
-    RC_(divide_conquer(E, s, &Z));
+    RC_(divide_conquer(E, s, &Z, at_noise));
     RC_(back_transform(E, Z, d_V, s));
     TSCF_CUDA_CHECK(cudaMemcpyAsync(d_w, E->pos.lam, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     return OK;

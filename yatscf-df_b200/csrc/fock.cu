@@ -14,6 +14,7 @@
 
 #include "tiles.cuh"
 #include "tscf_internal.h"
+#include "umma.cuh"
 
 namespace tscf {
 
@@ -182,11 +183,6 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, int by
     const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async16(double *dst, const double *src, int bytes)
-{
-    const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
@@ -194,9 +190,9 @@ struct KhCursor {
     int item, i, s0, p0, r0, r_end, step, nsteps;
 };
 
-template <int WS, int NX, int WP>
+template <int WS, int NX, int WP, int NY>
 struct KhTile {
-    static constexpr int S = WS * NX * 8, P = WP * 32, THREADS = WS * WP * 32;
+    static constexpr int S = WS * NX * 8, P = WP * NY * 8, THREADS = WS * WP * 32;
     static constexpr int AS = S + 4, BS = P + 4;   // strides = 4 or 12 (mod 16) doubles: conflict-free fragments
     static constexpr int STAGE = KT_K * (AS + BS);
     static constexpr size_t SMEM = sizeof(double) * KH_STAGES * STAGE;
@@ -228,21 +224,20 @@ __device__ __forceinline__ void kh_next(KhCursor &c, int n_items, int stiles, in
     else kh_set<S, P>(c, c.item + gridDim.x, n_items, stiles, ptiles, displs);
 }
 
-// VEC: 16-byte copies of the DF rows and stores of T (naux even, so every row starts 16-byte aligned)
-template <int WS, int NX, int WP, bool VEC>
-__global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
+// For an odd naux (rows start at any 8 bytes): every thread copies its share.
+template <int WS, int NX, int WP, int NY>
+__global__ void __launch_bounds__(KhTile<WS, NX, WP, NY>::THREADS, 1)
     k_halftransform_pipe(const double *__restrict__ B, const double *__restrict__ C, const int *__restrict__ csr_j,
                          const int *__restrict__ csr_u, const int *__restrict__ displs, int nocc, int naux,
                          double *__restrict__ T, int n_items, int stiles, int ptiles, unsigned long long *rowmax)
 {
-    using K = KhTile<WS, NX, WP>;
+    using K = KhTile<WS, NX, WP, NY>;
     constexpr int S = K::S, PW = K::P, NT = K::THREADS;
     extern __shared__ __align__(16) double khsm[];
-    constexpr int BCOPY = VEC ? 2 : 1;                      // doubles per B copy
-    constexpr int NBC = KT_K * PW / BCOPY, NB = (NBC + NT - 1) / NT;   // B copies per step, per thread
+    constexpr int NBC = KT_K * PW, NB = (NBC + NT - 1) / NT;   // B copies per step, per thread
     constexpr int NAC = KT_K * S, NA = (NAC + NT - 1) / NT;            // Cocc copies per step, per thread
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ws = (warp / WP) * NX * 8, wp = (warp % WP) * 32;
+    const int ws = (warp / WP) * NX * 8, wp = (warp % WP) * NY * 8;
     const int fr = lane >> 2, fc = lane & 3;
     int iu[NB], ij[NA];
     KhCursor P, Q;   // P: the next step to copy; Q: the step the tiles consume
@@ -252,7 +247,7 @@ __global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
 #pragma unroll
         for (int q = 0; q < NB; q++) {
             const int c = tid + NT * q;
-            const int r = P.r0 + c / (PW / BCOPY);
+            const int r = P.r0 + c / PW;
             iu[q] = (c < NBC && P.item < n_items && r < P.r_end) ? csr_u[r] : -1;
         }
 #pragma unroll
@@ -269,12 +264,11 @@ __global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
             for (int q = 0; q < NB; q++) {
                 const int c = tid + NT * q;
                 if (NBC % NT == 0 || c < NBC) {
-                    const int kk = c / (PW / BCOPY), cc = (c % (PW / BCOPY)) * BCOPY;
+                    const int kk = c / PW, cc = c % PW;
                     const int pg = P.p0 + cc;
                     const bool ok = iu[q] >= 0 && pg < naux;
                     const double *src = ok ? B + (size_t) iu[q] * naux + pg : B;
-                    if (VEC) cp_async16(&Bs[kk * K::BS + cc], src, ok ? 16 : 0);
-                    else cp_async8(&Bs[kk * K::BS + cc], src, ok ? 8 : 0);
+                    cp_async8(&Bs[kk * K::BS + cc], src, ok ? 8 : 0);
                 }
             }
 #pragma unroll
@@ -295,22 +289,22 @@ __global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
         kh_next<S, PW>(P, n_items, stiles, ptiles, displs);
     }
     load_idx();
-    double acc[NX][4][2];
+    double acc[NX][NY][2];
 #pragma unroll
     for (int x = 0; x < NX; x++)
 #pragma unroll
-        for (int y = 0; y < 4; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
+        for (int y = 0; y < NY; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
     for (int g = 0; Q.item < n_items; g++) {
         cp_async_wait<KH_STAGES - 2>();   // this thread's copies of step g have landed
         __syncthreads();                  // everyone's have, and step g - 1's buffer is free
         const double *As = khsm + (size_t) (g % KH_STAGES) * K::STAGE + fc * K::AS + ws + fr;
         const double *Bs = khsm + (size_t) (g % KH_STAGES) * K::STAGE + KT_K * K::AS + fc * K::BS + wp + fr;
-        double a[2][NX], b[2][4];
+        double a[2][NX], b[2][NY];
         auto frag = [&](int w, int k4) {
 #pragma unroll
             for (int x = 0; x < NX; x++) a[w][x] = As[k4 * K::AS + 8 * x];
 #pragma unroll
-            for (int y = 0; y < 4; y++) b[w][y] = Bs[k4 * K::BS + 8 * y];
+            for (int y = 0; y < NY; y++) b[w][y] = Bs[k4 * K::BS + 8 * y];
         };
         frag(0, 0);
 #pragma unroll
@@ -320,7 +314,7 @@ __global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
 #pragma unroll
             for (int x = 0; x < NX; x++)
 #pragma unroll
-                for (int y = 0; y < 4; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], a[w][x], b[w][y]);
+                for (int y = 0; y < NY; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], a[w][x], b[w][y]);
             if (k4 == 0) {   // the next copies go out behind the first DMMAs
                 issue((g + KH_STAGES - 1) % KH_STAGES);
                 kh_next<S, PW>(P, n_items, stiles, ptiles, displs);
@@ -334,15 +328,10 @@ __global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
                 const int sg = Q.s0 + ws + 8 * x + fr;
                 double *row = T + ((size_t) Q.i * nocc + (sg < nocc ? sg : 0)) * naux;
 #pragma unroll
-                for (int y = 0; y < 4; y++) {
+                for (int y = 0; y < NY; y++) {
                     const int pg = Q.p0 + wp + 8 * y + 2 * fc;
-                    if (VEC) {
-                        if (sg < nocc && pg < naux)
-                            *reinterpret_cast<double2 *>(row + pg) = make_double2(acc[x][y][0], acc[x][y][1]);
-                    } else {
-                        if (sg < nocc && pg < naux) row[pg] = acc[x][y][0];
-                        if (sg < nocc && pg + 1 < naux) row[pg + 1] = acc[x][y][1];
-                    }
+                    if (sg < nocc && pg < naux) row[pg] = acc[x][y][0];
+                    if (sg < nocc && pg + 1 < naux) row[pg + 1] = acc[x][y][1];
                     amax = fmax(amax, fmax(fabs(acc[x][y][0]), fabs(acc[x][y][1])));
                     acc[x][y][0] = acc[x][y][1] = 0.0;
                 }
@@ -357,53 +346,230 @@ __global__ void __launch_bounds__(KhTile<WS, NX, WP>::THREADS, 1)
     cp_async_wait<0>();
 }
 
-template <int WS, int NX, int WP>
-static void launch_half_pipe(const FockPlan &p, const double *C, double *T, unsigned long long *rowmax, cudaStream_t s)
+// ---- the same tiles with a producer warp (even naux): it keeps bulk copies of
+// the chunks' rows in flight (one instruction a row, 16-byte aligned because
+// naux and the padded row pitch of Cocc are even) behind mbarriers, so the other
+// warps only read fragments and issue DMMAs, and drift apart by up to the
+// pipeline's depth: nothing but the chunk they wait for stops them. With all warps
+// issuing the copies between block barriers the tensor cores idled 30% of the
+// time (C40H82 13.4 ms, now 10.1 ms; C20H42 1.82 ms, now 1.40 ms). The copies in one
+// of the tiles' warps instead cost more than they saved (13.7 ms). The SM quarter
+// that holds the producer as its fourth warp gives each 128 registers, which
+// bounds the tile of 12 warps (56 x 24 a warp).
+constexpr long long KH_WAIT = 2000000000LL;   // clock cycles a barrier wait may take (~1 s)
+__device__ int g_half_error;
+
+__device__ __forceinline__ void bulk_row(double *dst, const double *src, unsigned bytes, uint64_t *bar)
 {
-    using K = KhTile<WS, NX, WP>;
-    const int stiles = (p.nocc + K::S - 1) / K::S, ptiles = (p.naux + K::P - 1) / K::P;
-    const long long items = (long long) p.nbf * stiles * ptiles;
-    auto go = [&](auto kernel) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) K::SMEM);
-        int per = 1;   // the small tiles fit several times on an SM
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, K::THREADS, K::SMEM);
-        const int grid = (int) std::min<long long>(items, (long long) num_sms() * std::max(per, 1));
-        kernel<<<grid, K::THREADS, K::SMEM, s>>>(p.B, C, p.csr_j, p.csr_u, p.csr_displs, p.nocc, p.naux, T, (int) items,
-                                                 stiles, ptiles, rowmax);
-    };
-    if (p.naux % 2 == 0) go(k_halftransform_pipe<WS, NX, WP, true>);
-    else go(k_halftransform_pipe<WS, NX, WP, false>);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     umma::smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(umma::smem_u32(bar))
+                 : "memory");
 }
 
-// The tile for n_occ: one row of warps up to 56 occupied orbitals, two up to
-// 112, three up to 168 and for the equal parts of more; wide: 256 or 192 aux
-// columns for the first two (fewer re-reads of Cocc), narrow: 128 (less padding
-// of a short aux dimension); the autotuner times both.
+template <int WS, int NX, int WP, int NY>
+struct KhBulk : KhTile<WS, NX, WP, NY> {
+    using K = KhTile<WS, NX, WP, NY>;
+    static constexpr int WARPS = WS * WP, THREADS = (WARPS + 1) * 32;
+    static constexpr int FIT = (int) ((220 << 10) / (sizeof(double) * K::STAGE));
+    static constexpr int STAGES = FIT < 6 ? FIT : 6;
+    static constexpr size_t SMEM = sizeof(double) * STAGES * K::STAGE;
+};
+
+// Cocc in rows of cp doubles (zeros behind n_occ), then a block of zeros for the rows behind a chunk's last.
+__global__ void k_pad_cocc(const double *__restrict__ C, double *__restrict__ Cp, int nbf, int nocc, int cp, int zeros)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nbf * cp + zeros) return;
+    const int i = k / cp, s = k - i * cp;
+    Cp[k] = (i < nbf && s < nocc) ? C[(size_t) i * nocc + s] : 0.0;
+}
+
+template <int WS, int NX, int WP, int NY>
+__global__ void __launch_bounds__(KhBulk<WS, NX, WP, NY>::THREADS, 1)
+    k_halftransform_bulk(const double *__restrict__ B, const double *__restrict__ Cp, int cp, const double *zeros,
+                         const int *__restrict__ csr_j, const int *__restrict__ csr_u, const int *__restrict__ displs,
+                         int nocc, int naux, double *__restrict__ T, int n_items, int stiles, int ptiles,
+                         unsigned long long *rowmax)
+{
+    using K = KhBulk<WS, NX, WP, NY>;
+    constexpr int S = K::S, PW = K::P, ST = K::STAGES;
+    extern __shared__ __align__(16) double khsm[];
+    __shared__ uint64_t full[ST], empty[ST];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        for (int k = 0; k < ST; k++) {
+            umma::mbar_init(&full[k], 1);
+            umma::mbar_init(&empty[k], K::WARPS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async;" ::: "memory");
+    }
+    __syncthreads();
+    KhCursor Q;
+    kh_set<S, PW>(Q, blockIdx.x, n_items, stiles, ptiles, displs);
+    if (warp == K::WARPS) {   // ---- producer: lanes 0..15 copy the chunk's DF rows, lanes 16..31 its rows of Cocc
+        const int kk = lane & 15;
+        const bool isB = lane < 16;
+        int idx = -1;
+        auto fetch = [&]() {
+            const int r = Q.r0 + kk;
+            idx = (Q.item < n_items && r < Q.r_end) ? (isB ? csr_u[r] : csr_j[r]) : -1;
+        };
+        fetch();
+        for (int g = 0; Q.item < n_items; g++) {
+            const int st = g % ST;
+            if (g >= ST && !umma::mbar_wait_bounded(&empty[st], ((g / ST) - 1) & 1, &g_half_error, 31, KH_WAIT)) {
+                for (int k = g - ST; k < g; k++)   // its copies in flight
+                    umma::mbar_wait_bounded(&full[k % ST], (k / ST) & 1, &g_half_error, 32, KH_WAIT);
+                return;
+            }
+            double *As = khsm + (size_t) st * K::STAGE, *Bs = As + KT_K * K::AS;
+            const unsigned nb = (unsigned) min(PW, naux - Q.p0) * 8u, na = S * 8u;
+            if (lane == 0) umma::mbar_expect_tx(&full[st], KT_K * (nb + na));
+            __syncwarp();
+            if (isB) bulk_row(Bs + kk * K::BS, idx >= 0 ? B + (size_t) idx * naux + Q.p0 : zeros, nb, &full[st]);
+            else bulk_row(As + kk * K::AS, idx >= 0 ? Cp + (size_t) idx * cp + Q.s0 : zeros, na, &full[st]);
+            kh_next<S, PW>(Q, n_items, stiles, ptiles, displs);
+            fetch();
+        }
+        return;
+    }
+    const int ws = (warp / WP) * NX * 8, wp = (warp % WP) * NY * 8;
+    const int fr = lane >> 2, fc = lane & 3;
+    double acc[NX][NY][2];
+#pragma unroll
+    for (int x = 0; x < NX; x++)
+#pragma unroll
+        for (int y = 0; y < NY; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
+    int st = 0, phase = 0;
+    while (Q.item < n_items) {
+        if (!umma::mbar_wait_bounded(&full[st], phase, &g_half_error, 33, KH_WAIT)) return;
+        const double *As = khsm + (size_t) st * K::STAGE + fc * K::AS + ws + fr;
+        const double *Bs = khsm + (size_t) st * K::STAGE + KT_K * K::AS + fc * K::BS + wp + fr;
+#pragma unroll
+        for (int k4 = 0; k4 < KT_K; k4 += 4) {
+            double a[NX], b[NY];
+#pragma unroll
+            for (int x = 0; x < NX; x++) a[x] = As[k4 * K::AS + 8 * x];
+#pragma unroll
+            for (int y = 0; y < NY; y++) b[y] = Bs[k4 * K::BS + 8 * y];
+#pragma unroll
+            for (int x = 0; x < NX; x++)
+#pragma unroll
+                for (int y = 0; y < NY; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], a[x], b[y]);
+        }
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(&empty[st]);
+        if (++st == ST) {
+            st = 0;
+            phase ^= 1;
+        }
+        if (++Q.step < Q.nsteps) continue;
+        double amax = 0.0;   // item done: write its tile, start the next
+#pragma unroll
+        for (int x = 0; x < NX; x++) {
+            const int sg = Q.s0 + ws + 8 * x + fr;
+            double *row = T + ((size_t) Q.i * nocc + (sg < nocc ? sg : 0)) * naux;
+#pragma unroll
+            for (int y = 0; y < NY; y++) {
+                const int pg = Q.p0 + wp + 8 * y + 2 * fc;
+                if (sg < nocc && pg < naux) {
+                    *reinterpret_cast<double2 *>(row + pg) = make_double2(acc[x][y][0], acc[x][y][1]);
+                    amax = fmax(amax, fmax(fabs(acc[x][y][0]), fabs(acc[x][y][1])));
+                }
+                acc[x][y][0] = acc[x][y][1] = 0.0;
+            }
+        }
+        if (rowmax) {
+            for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffff, amax, o));
+            if (lane == 0 && amax > 0.0) atomicMax(rowmax + Q.i, (unsigned long long) __double_as_longlong(amax));
+        }
+        kh_set<S, PW>(Q, Q.item + gridDim.x, n_items, stiles, ptiles, displs);
+    }
+}
+
+int half_error_flag()
+{
+    int v = 0;
+    cudaMemcpyFromSymbol(&v, g_half_error, sizeof(int));
+    return v;
+}
+
+// Doubles of FockPlan::Cpad for nbf x nocc: rows padded to whole tiles, and a block of zeros.
+size_t half_pad_elems(int nbf, int nocc)
+{
+    const size_t tiles = (nocc + KH_SMAX - 1) / KH_SMAX;
+    return (size_t) nbf * (nocc + 32 * tiles) + 512;
+}
+
+template <int WS, int NX, int WP, int NY>
+static void launch_half(const FockPlan &p, const double *C, double *T, unsigned long long *rowmax, cudaStream_t s)
+{
+    using K = KhTile<WS, NX, WP, NY>;
+    using KB = KhBulk<WS, NX, WP, NY>;
+    const int stiles = (p.nocc + K::S - 1) / K::S, ptiles = (p.naux + K::P - 1) / K::P;
+    const long long items = (long long) p.nbf * stiles * ptiles;
+    auto grid = [&](auto kernel, int threads, size_t smem) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        int per = 1;   // the small tiles fit several times on an SM
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
+        return (int) std::min<long long>(items, (long long) num_sms() * std::max(per, 1));
+    };
+    if (p.naux % 2 == 0 && p.Cpad) {
+        const int cp = stiles * K::S, zeros = std::max(K::S, K::P);
+        const int n = p.nbf * cp + zeros;
+        k_pad_cocc<<<(n + 255) / 256, 256, 0, s>>>(C, p.Cpad, p.nbf, p.nocc, cp, zeros);
+        g_launches++;
+        const int g = grid(k_halftransform_bulk<WS, NX, WP, NY>, KB::THREADS, KB::SMEM);
+        k_halftransform_bulk<WS, NX, WP, NY><<<g, KB::THREADS, KB::SMEM, s>>>(
+            p.B, p.Cpad, cp, p.Cpad + (size_t) p.nbf * cp, p.csr_j, p.csr_u, p.csr_displs, p.nocc, p.naux, T,
+            (int) items, stiles, ptiles, rowmax);
+    } else {
+        const int g = grid(k_halftransform_pipe<WS, NX, WP, NY>, K::THREADS, K::SMEM);
+        k_halftransform_pipe<WS, NX, WP, NY><<<g, K::THREADS, K::SMEM, s>>>(p.B, C, p.csr_j, p.csr_u, p.csr_displs, p.nocc,
+                                                                        p.naux, T, (int) items, stiles, ptiles, rowmax);
+    }
+}
+
+// The tile for the occupied part o (n_occ in equal parts of at most 168): the
+// fewest padded orbitals within the registers, 4 warps or a multiple (each SM
+// quarter has its own FP64 tensor pipe: 9 warps of 56 x 32 took 13.0 ms on C40H82).
+//   o <= 56:  one row of warps, 8 o' x 32 outputs a warp; 128 or 256 aux columns
+//   o <= 88:  one row, 24 aux columns a warp, 192 in all; or two rows, 128 columns
+//   o <= 128: two rows, 128 columns
+//   o <= 168: three rows, 12 warps: 96 columns without, or 128 with spilled registers
+// Where two are named the autotuner times both.
 static void half_pipe(const FockPlan &p, const double *C, double *T, unsigned long long *rowmax, cudaStream_t s, bool wide)
 {
     const int tiles = (p.nocc + KH_SMAX - 1) / KH_SMAX, o = (p.nocc + tiles - 1) / tiles;
-    const int ws = o <= 56 ? 1 : (o <= 112 ? 2 : 3), nx = (o + 8 * ws - 1) / (8 * ws);
-#define TSCF_HALF(WS, NX, WIDE)                                          \
-    case 10 * WS + NX:                                                   \
-        if (wide) launch_half_pipe<WS, NX, WIDE>(p, C, T, rowmax, s);    \
-        else launch_half_pipe<WS, NX, 4>(p, C, T, rowmax, s);            \
-        break;
-    switch (10 * ws + nx) {
-        TSCF_HALF(1, 1, 8)
-        TSCF_HALF(1, 2, 8)
-        TSCF_HALF(1, 3, 8)
-        TSCF_HALF(1, 4, 8)
-        TSCF_HALF(1, 5, 8)
-        TSCF_HALF(1, 6, 8)
-        TSCF_HALF(1, 7, 8)
-        TSCF_HALF(2, 4, 6)
-        TSCF_HALF(2, 5, 6)
-        TSCF_HALF(2, 6, 6)
-        TSCF_HALF(2, 7, 6)
-        TSCF_HALF(3, 5, 4)
-        TSCF_HALF(3, 6, 4)
-        TSCF_HALF(3, 7, 4)
-    default: break;   // none left: a part of n_occ in 1..56, 57..112 or 113..168 has these NX
+#define TSCF_HALF(WS, NX, WP, NY)                       \
+    case NX:                                            \
+        launch_half<WS, NX, WP, NY>(p, C, T, rowmax, s); \
+        return;
+    if (o <= 56 && !wide) {
+        switch ((o + 7) / 8) {
+            TSCF_HALF(1, 1, 4, 4) TSCF_HALF(1, 2, 4, 4) TSCF_HALF(1, 3, 4, 4) TSCF_HALF(1, 4, 4, 4)
+            TSCF_HALF(1, 5, 4, 4) TSCF_HALF(1, 6, 4, 4) TSCF_HALF(1, 7, 4, 4)
+        }
+    } else if (o <= 56) {
+        switch ((o + 7) / 8) {
+            TSCF_HALF(1, 1, 8, 4) TSCF_HALF(1, 2, 8, 4) TSCF_HALF(1, 3, 8, 4) TSCF_HALF(1, 4, 8, 4)
+            TSCF_HALF(1, 5, 8, 4) TSCF_HALF(1, 6, 8, 4) TSCF_HALF(1, 7, 8, 4)
+        }
+    } else if (o <= 88 && wide) {
+        switch ((o + 7) / 8) {
+            TSCF_HALF(1, 8, 8, 3) TSCF_HALF(1, 9, 8, 3) TSCF_HALF(1, 10, 8, 3) TSCF_HALF(1, 11, 8, 3)
+        }
+    } else if (o <= 128) {
+        switch ((o + 15) / 16) {
+            TSCF_HALF(2, 4, 4, 4) TSCF_HALF(2, 5, 4, 4) TSCF_HALF(2, 6, 4, 4) TSCF_HALF(2, 7, 4, 4)
+            TSCF_HALF(2, 8, 4, 4)
+        }
+    } else if (!wide) {
+        switch ((o + 23) / 24) { TSCF_HALF(3, 6, 4, 3) TSCF_HALF(3, 7, 4, 3) }
+    } else {
+        switch ((o + 23) / 24) { TSCF_HALF(3, 6, 4, 4) TSCF_HALF(3, 7, 4, 4) }
     }
 #undef TSCF_HALF
 }

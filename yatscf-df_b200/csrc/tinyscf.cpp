@@ -305,6 +305,7 @@ struct Engine {
     double *B = nullptr;
     int aux_p0 = 0, aux_ns = 0;   // aux columns [aux_p0, aux_p0 + aux_ns) of the DF tensor held (0: all)
     double *T = nullptr, *Kpart = nullptr;
+    double *Cpad = nullptr;       // Cocc in padded rows, for the half-transform
     int2 *tiles = nullptr;
     int ksplit = 1, ksplit_max = 1, ksplit64 = 1, ktile = 64, khwide = 0;
     int2 *tiles128 = nullptr;
@@ -362,6 +363,7 @@ struct Engine {
         p.up_j = up_j;
         p.up_u = up_u;
         p.B = B;
+        p.Cpad = Cpad;
         return p;
     }
 };
@@ -924,6 +926,7 @@ int sparsity_impl(TinySCF_t t)
     // DF tensor, K and J buffers
     RC(dalloc(e, &e->B, (size_t) nu * naux));
     RC(dalloc(e, &e->T, (size_t) nbf * nocc * naux));
+    RC(dalloc(e, &e->Cpad, half_pad_elems(nbf, nocc)));
     const int nt = (nbf + 63) / 64, ntiles = nt * (nt + 1) / 2;
     const int nt2 = (nbf + 127) / 128, ntiles2 = nt2 * (nt2 + 1) / 2;
     const int nsm = num_sms();
@@ -1414,7 +1417,7 @@ int density_device(TinySCF_t t)
             return cuda_rc("density (subspace refinement)");
         }
     }
-    RC(eig_run(e->eig, Fo, e->w, e->V, e->s));
+    RC(eig_run(e->eig, Fo, e->w, e->V, e->s, e->dmode != TINYSCF_DENSITY_REFINE));
     { density_from_eig(e->X, e->V, e->Cocc, e->D, n, o, e->s); e->d_from_cocc = true; }
     e->n_eig++;
     if (e->dmode == TINYSCF_DENSITY_REFINE && o > 0) {
@@ -1680,6 +1683,10 @@ int scf_impl(TinySCF_t t)
             fprintf(stderr, "[tinyscf] tensor-core K: a bounded wait timed out (code %d)\n", fl);
             return ERR_CUDA;
         }
+    }
+    if (const int fl = half_error_flag()) {
+        fprintf(stderr, "[tinyscf] exchange half-transform: a bounded wait timed out (code %d)\n", fl);
+        return ERR_CUDA;
     }
     if (e->oz) {
         const int fl = oz_error_flag();
@@ -2373,7 +2380,9 @@ int batch_eigs(TinySCF_batch_t b, const std::vector<int> &need)
     for (auto &g : b->groups) {
         const int64_t cnt = (int64_t) g.members.size(), n = g.n;
         for (int64_t k = 0; k < cnt; k++)
-            if (need[g.members[k]]) RC(eig_run(g.eig, g.A + k * n * n, g.W + k * n, g.A + k * n * n, b->s));
+            if (need[g.members[k]])
+                RC(eig_run(g.eig, g.A + k * n * n, g.W + k * n, g.A + k * n * n, b->s,
+                           E_(b->mols[g.members[k]])->dmode != TINYSCF_DENSITY_REFINE));
     }
     return OK;
 }
@@ -2700,7 +2709,7 @@ int TinySCF_eigh(int device, int n, const double *A, double *w, double *V)
     } else if (cudaMemcpyAsync(dA, A, sizeof(double) * nn, cudaMemcpyHostToDevice, s) != cudaSuccess) {
         rc = TINYSCF_ERR_CUDA;
     } else {
-        rc = eig_run(eg, dA, dw, dV, s);
+        rc = eig_run(eg, dA, dw, dV, s, true);
         if (rc == OK && (cudaMemcpyAsync(w, dw, sizeof(double) * n, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaMemcpyAsync(V, dV, sizeof(double) * nn, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaStreamSynchronize(s) != cudaSuccess))

@@ -151,7 +151,8 @@ constexpr int EIG_MAX_N = 8192;
 struct Eig;
 Eig *eig_create(int n, cudaStream_t s);
 void eig_destroy(Eig *e);
-int  eig_run(Eig *e, const double *d_A, double *d_w, double *d_V, cudaStream_t s);
+// at_noise: the secular equation's roots stop where its value is rounding (k_dc_secular).
+int  eig_run(Eig *e, const double *d_A, double *d_w, double *d_V, cudaStream_t s, bool at_noise = false);
 int  eig_error(Eig *e);
 
 // Orthonormal rows U (o x n) spanning the dominant o-dimensional invariant
@@ -189,6 +190,7 @@ struct FockPlan {
     const int *up_i, *up_j;   // [nup] upper CSR entries (i <= j)
     const int *up_u;          // [nup] their unique-pair rows
     const double *B;          // DF tensor, [nu][naux] unique pairs
+    double *Cpad;             // half_pad_elems(nbf, nocc) doubles of scratch, or nullptr
 };
 // J = symmetrised Coulomb matrix from D (build_Fock.c:37-130).
 // d_t (naux) and d_part (scratch, nblk*naux) are caller buffers.
@@ -209,6 +211,8 @@ void convert_f32(const double *in, float *out, size_t n, cudaStream_t s);
 // double bits, for the integer-tensor-core K.
 void build_K_halftransform(const FockPlan &p, const double *d_Cocc, double *d_T, cudaStream_t s, int wide = 0,
                            unsigned long long *d_rowmax = nullptr);
+size_t half_pad_elems(int nbf, int nocc);
+int    half_error_flag();   // nonzero: a bounded wait of the half-transform gave up
 // ... then K = T T^T over upper 64x64 tiles (d_tiles: (bi,bj), bi <= bj), split-K, mirrored.
 // tile = 64 (k_syrk_part, FFMA), 128 (k_syrk_part128, FFMA) or KSYRK_DMMA
 // (k_syrk_dmma: 128 x 128 tiles on the FP64 tensor cores); d_tiles lists the
