@@ -970,6 +970,60 @@ __global__ void k_dc_init(const double *d, const double *e, double *lam, double 
     Qb[(size_t) i * n + i] = 1.0;
 }
 
+// The deflation scan of a merge, by one thread: small z components, and close
+// pairs that a Givens rotation deflates (LAPACK dlaed2's two tests). sd, sz are
+// the sorted d and z (modified by the rotations).
+__device__ __forceinline__ void deflation_scan(double *sd, double *sz, int m, double rho, double zmax, double tol,
+                                               int *keep, int *defl, int *rowinfo, int2 *rot, double2 *rotcs, int &k,
+                                               int &nr)
+{
+    int nd_ = 0;
+    k = nr = 0;
+    if (rho * zmax <= tol) {
+        for (int s = 0; s < m; s++) {
+            rowinfo[s] = -(nd_ + 1);
+            defl[nd_++] = s;
+        }
+    } else {
+        int pj = -1;
+        for (int s = 0; s < m; s++) {
+            if (rho * fabs(sz[s]) <= tol) {
+                rowinfo[s] = -(nd_ + 1);
+                defl[nd_++] = s;
+                continue;
+            }
+            if (pj < 0) {
+                pj = s;
+                continue;
+            }
+            // close pair: |t C S| <= tol with C = z_s / h, S = -z_pj / h, h = hypot(z_s, z_pj)
+            const double zp = sz[pj], zs = sz[s], t = sd[s] - sd[pj];
+            if (fabs(t * zs * zp) <= tol * (zs * zs + zp * zp)) {
+                const double tt = hypot(zs, zp), C = zs / tt, S = -zp / tt;
+                sz[s] = tt;
+                sz[pj] = 0.0;
+                rot[nr] = make_int2(pj, s);
+                rotcs[nr] = make_double2(C, S);
+                nr++;
+                const double dp = sd[pj] * C * C + sd[s] * S * S;
+                sd[s] = sd[pj] * S * S + sd[s] * C * C;
+                sd[pj] = dp;
+                rowinfo[pj] = -(nd_ + 1);
+                defl[nd_++] = pj;
+                pj = s;
+            } else {
+                rowinfo[pj] = k;
+                keep[k++] = pj;
+                pj = s;
+            }
+        }
+        if (pj >= 0) {
+            rowinfo[pj] = k;
+            keep[k++] = pj;
+        }
+    }
+}
+
 // Sorting of the two halves, z, the tolerance and the deflation scan. One CTA per node.
 __global__ void __launch_bounds__(512) k_dc_deflate(DcNodes nd, DcPos ps, const double *Q, const double *e, int n,
                                                     int node0)
@@ -1029,50 +1083,8 @@ __global__ void __launch_bounds__(512) k_dc_deflate(DcNodes nd, DcPos ps, const 
     const double tol = 8.0 * DBL_EPSILON * fmax(dmax, zmax);
     int *keep = ps.keep + lo, *defl = ps.defl + lo, *rowinfo = ps.rowinfo + lo;
     if (threadIdx.x == 0) {
-        int k = 0, nd_ = 0, nr = 0;
-        if (rho * zmax <= tol) {
-            for (int s = 0; s < m; s++) {
-                rowinfo[s] = -(nd_ + 1);
-                defl[nd_++] = s;
-            }
-        } else {
-            int pj = -1;
-            for (int s = 0; s < m; s++) {
-                if (rho * fabs(sz[s]) <= tol) {
-                    rowinfo[s] = -(nd_ + 1);
-                    defl[nd_++] = s;
-                    continue;
-                }
-                if (pj < 0) {
-                    pj = s;
-                    continue;
-                }
-                // close pair: |t C S| <= tol with C = z_s / h, S = -z_pj / h, h = hypot(z_s, z_pj)
-                const double zp = sz[pj], zs = sz[s], t = sd[s] - sd[pj];
-                if (fabs(t * zs * zp) <= tol * (zs * zs + zp * zp)) {
-                    const double tt = hypot(zs, zp), C = zs / tt, S = -zp / tt;
-                    sz[s] = tt;
-                    sz[pj] = 0.0;
-                    ps.rot[lo + nr] = make_int2(pj, s);
-                    ps.rotcs[lo + nr] = make_double2(C, S);
-                    nr++;
-                    const double dp = sd[pj] * C * C + sd[s] * S * S;
-                    sd[s] = sd[pj] * S * S + sd[s] * C * C;
-                    sd[pj] = dp;
-                    rowinfo[pj] = -(nd_ + 1);
-                    defl[nd_++] = pj;
-                    pj = s;
-                } else {
-                    rowinfo[pj] = k;
-                    keep[k++] = pj;
-                    pj = s;
-                }
-            }
-            if (pj >= 0) {
-                rowinfo[pj] = k;
-                keep[k++] = pj;
-            }
-        }
+        int k, nr;
+        deflation_scan(sd, sz, m, rho, zmax, tol, keep, defl, rowinfo, ps.rot + lo, ps.rotcs + lo, k, nr);
         nd.kcnt[node] = k;
         nd.rcnt[node] = nr;
         nd.rho[node] = rho;
@@ -1129,23 +1141,10 @@ __device__ __forceinline__ void secular_parts(const double *sd, const double *sz
 // as far as f can (the criterion of LAPACK's dlaed4): 13 us. The bracketed
 // stop stays for the eigenbases of the accelerated form and of X and (P|Q)^-1/2,
 // whose users amplify the last bits (1e-16 in X moves its density by 1e-9).
-__global__ void __launch_bounds__(256) k_dc_secular(DcNodes nd, DcPos ps, const int2 *tab, bool at_noise)
+// One warp; the root of position j as org, tau (tau relative to sd[org]).
+__device__ __forceinline__ void secular_root(const double *sd, const double *sz, int k, int j, double rho, int lane,
+                                             bool at_noise, int &org, double &tau)
 {
-    extern __shared__ double dsm[];
-    const int2 tb = tab[blockIdx.x];
-    const int node = tb.x, lo = nd.lo[node], k = nd.kcnt[node];
-    if (tb.y >= k) return;
-    double *sd = dsm, *sz = dsm + k;
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        sd[i] = ps.dK[lo + i];
-        sz[i] = ps.zK[lo + i];
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, j = tb.y + (threadIdx.x >> 5);
-    if (j >= k) return;
-    const double rho = nd.rho[node];
-    int org;
-    double tau;
     if (k == 1) {
         org = 0;
         tau = rho * sz[0] * sz[0];
@@ -1214,6 +1213,26 @@ __global__ void __launch_bounds__(256) k_dc_secular(DcNodes nd, DcPos ps, const 
             if (done) break;
         }
     }
+}
+
+__global__ void __launch_bounds__(256) k_dc_secular(DcNodes nd, DcPos ps, const int2 *tab, bool at_noise)
+{
+    extern __shared__ double dsm[];
+    const int2 tb = tab[blockIdx.x];
+    const int node = tb.x, lo = nd.lo[node], k = nd.kcnt[node];
+    if (tb.y >= k) return;
+    double *sd = dsm, *sz = dsm + k;
+    for (int i = threadIdx.x; i < k; i += blockDim.x) {
+        sd[i] = ps.dK[lo + i];
+        sz[i] = ps.zK[lo + i];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, j = tb.y + (threadIdx.x >> 5);
+    if (j >= k) return;
+    const double rho = nd.rho[node];
+    int org;
+    double tau;
+    secular_root(sd, sz, k, j, rho, lane, at_noise, org, tau);
     if (lane == 0) {
         ps.lamb[lo + j] = sd[org];
         ps.tau[lo + j] = tau;
@@ -1358,6 +1377,162 @@ __global__ void __launch_bounds__(128) k_dc_gemm(DcNodes nd, const int4 *tiles, 
     const double *Bb = Us + (size_t) r0 * n + lo;
     double *Cb = Qout + (size_t) r0 * n + lo;
     dgemm_tile_dmma64<false, false>(mh, m, mh, 1.0, Ab, n, Bb, n, 0.0, Cb, n, t.y * 64, t.z * 64);
+}
+
+// A merge of at most DC_SMALL positions in one CTA: the nine steps above in
+// shared memory, one launch per tree level instead of nine (the levels below 64
+// were 54 of an eigensolve's launches, each a few us for almost no work). Every
+// value is formed as in the separate kernels: the same bits.
+constexpr int DC_SMALL = 64;
+constexpr size_t DC_SMALL_SMEM = sizeof(double) * DC_SMALL * (DC_SMALL + 1 + DC_SMALL / 2 + 1);
+__global__ void __launch_bounds__(256) k_dc_merge_small(DcNodes nd, double *lam, const double *e, const double *Qin,
+                                                        double *Qout, int n, int node0, bool at_noise)
+{
+    constexpr int MS = DC_SMALL;
+    __shared__ double sd[MS], sz[MS], dK[MS], zK[MS], lamb[MS], tau[MS], zh[MS], nrm[MS], sv[MS], s_red[33];
+    __shared__ int sp[MS], keep[MS], defl[MS], rowinfo[MS], colsrc[MS];
+    __shared__ int2 rot[MS];
+    __shared__ double2 rotcs[MS];
+    __shared__ int s_k, s_nr;
+    extern __shared__ double dsm[];
+    double (*U)[MS + 1] = (double (*)[MS + 1]) dsm;
+    double (*Q)[MS / 2 + 1] = (double (*)[MS / 2 + 1]) (dsm + MS * (MS + 1));   // both halves' vectors, row by row
+    const int node = node0 + blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int lo = nd.lo[node], mid = nd.mid[node], hi = nd.hi[node];
+    const int m = hi - lo, m1 = mid - lo, m2 = hi - mid;
+    const double rho_raw = e[mid - 1];
+    const double rho = 2.0 * fabs(rho_raw), sg = rho_raw >= 0.0 ? 1.0 : -1.0;
+    const double *L1 = lam + lo, *L2 = lam + mid;
+    const double rs2 = 1.0 / sqrt(2.0);
+    for (int l = tid; l < m * (MS / 2); l += 256) {
+        const int i = l / (MS / 2), c = l % (MS / 2), r0 = i < m1 ? lo : mid, mh = i < m1 ? m1 : m2;
+        if (c < mh) Q[i][c] = Qin[(size_t) (lo + i) * n + r0 + c];
+    }
+    for (int idx = tid; idx < m; idx += 256) {
+        sd[idx] = 0.0;
+        sz[idx] = 0.0;
+        sp[idx] = idx;
+        colsrc[idx] = 0;
+    }
+    __syncthreads();
+    // sorting of the halves, z, tolerance
+    double dmax = 0.0, zmax = 0.0;
+    for (int idx = tid; idx < m; idx += 256) {
+        double x, zz;
+        int pos;
+        if (idx < m1) {
+            x = L1[idx];
+            zz = Q[m1 - 1][idx];
+            int a = 0, b = m2;   // first L2 >= x
+            while (a < b) {
+                const int c = (a + b) >> 1;
+                if (L2[c] < x) a = c + 1; else b = c;
+            }
+            pos = idx + a;
+        } else {
+            const int i2 = idx - m1;
+            x = L2[i2];
+            zz = sg * Q[m1][i2];
+            int a = 0, b = m1;   // first L1 > x
+            while (a < b) {
+                const int c = (a + b) >> 1;
+                if (L1[c] <= x) a = c + 1; else b = c;
+            }
+            pos = i2 + a;
+        }
+        pos = min(max(pos, 0), m - 1);
+        zz *= rs2;
+        sd[pos] = x;
+        sz[pos] = zz;
+        sp[pos] = idx;
+        dmax = fmax(dmax, fabs(x));
+        zmax = fmax(zmax, fabs(zz));
+    }
+    dmax = block_max_all<256>(dmax, s_red);
+    zmax = block_max_all<256>(zmax, s_red);
+    const double tol = 8.0 * DBL_EPSILON * fmax(dmax, zmax);
+    if (tid == 0) {
+        int k, nr;
+        deflation_scan(sd, sz, m, rho, zmax, tol, keep, defl, rowinfo, rot, rotcs, k, nr);
+        s_k = k;
+        s_nr = nr;
+    }
+    __syncthreads();
+    const int k = s_k, nr = s_nr;
+    for (int i = tid; i < k; i += 256) {
+        dK[i] = sd[keep[i]];
+        zK[i] = sz[keep[i]];
+    }
+    __syncthreads();
+    for (int j = wid; j < k; j += 8) {   // roots
+        int org;
+        double t;
+        secular_root(dK, zK, k, j, rho, lane, at_noise, org, t);
+        if (lane == 0) {
+            lamb[j] = dK[org];
+            tau[j] = t;
+        }
+    }
+    __syncthreads();
+    for (int i = wid; i < k; i += 8) {   // z from the roots
+        const double di = dK[i];
+        double pr = 1.0;
+        for (int j = lane; j < k; j += 32) {
+            const double del = (di - lamb[j]) - tau[j];
+            pr *= (j == i) ? del : del / (di - dK[j]);
+        }
+        pr = warp_prod_bcast(pr);
+        if (lane == 0) zh[i] = copysign(sqrt(fmax(-pr, 0.0)), zK[i]);
+    }
+    __syncthreads();
+    for (int j = wid; j < k; j += 8) {   // norms
+        const double lb = lamb[j], tj = tau[j];
+        double q = 0.0;
+        for (int i = lane; i < k; i += 32) {
+            const double u = zh[i] / ((dK[i] - lb) - tj);
+            q += u * u;
+        }
+        q = warp_sum_bcast(q);
+        if (lane == 0) nrm[j] = sqrt(q);
+    }
+    for (int a = tid; a < m; a += 256) sv[a] = (a < k) ? lamb[a] + tau[a] : sd[defl[a - k]];
+    __syncthreads();
+    if (tid < m) {   // output order
+        const double x = sv[tid];
+        int q = 0;
+        for (int b = 0; b < m; b++) {
+            const double y = sv[b];
+            q += (y < x || (y == x && b < tid)) ? 1 : 0;
+        }
+        q = min(q, m - 1);
+        lam[lo + q] = x;   // every read of the halves' values lies behind a barrier
+        colsrc[q] = tid;
+    }
+    __syncthreads();
+    for (int l = tid; l < m * m; l += 256) {   // the merge's vectors, in the children's order
+        const int sidx = l / m, c = l - sidx * m;
+        const int info = rowinfo[sidx], src = colsrc[c];
+        double v;
+        if (src < k) v = info >= 0 ? zh[info] / ((dK[info] - lamb[src]) - tau[src]) / nrm[src] : 0.0;
+        else v = (info < 0 && -(info + 1) == src - k) ? 1.0 : 0.0;
+        U[sp[sidx]][c] = v;
+    }
+    __syncthreads();
+    if (tid < m)
+        for (int q = nr - 1; q >= 0; q--) {
+            const int ix = sp[rot[q].x], iy = sp[rot[q].y];
+            const double2 cs = rotcs[q];
+            const double x = U[ix][tid], y = U[iy][tid];
+            U[ix][tid] = cs.x * x - cs.y * y;
+            U[iy][tid] = cs.y * x + cs.x * y;
+        }
+    __syncthreads();
+    for (int l = tid; l < m * m; l += 256) {   // [Q1 0; 0 Q2] U: one chain of multiply-adds per output, as DMMA
+        const int i = l / m, c = l - i * m, b0 = i < m1 ? 0 : m1, mh = i < m1 ? m1 : m2;
+        double acc = 0.0;
+        for (int q = 0; q < mh; q++) acc = fma(Q[i][q], U[b0 + q][c], acc);
+        Qout[(size_t) (lo + i) * n + lo + c] = acc;
+    }
 }
 
 __global__ void k_transpose(const double *in, double *out, int n)
@@ -1579,7 +1754,7 @@ bool smem_optin()
     if (done_dev == dev) return true;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
     if (!optin_one(k_sytrd_panel, optin) || !optin_one(k_wy_tfactor, optin) || !optin_one(k_dc_deflate, optin) ||
-        !optin_one(k_dc_secular, optin) ||
+        !optin_one(k_dc_merge_small, optin) || !optin_one(k_dc_secular, optin) ||
         !optin_one(k_dc_zhat, optin) || !optin_one(k_dc_norms, optin) || !optin_one(k_dc_order, optin))
         return false;
     done_dev = dev;
@@ -1733,6 +1908,12 @@ int divide_conquer(Eig *E, cudaStream_t s, double **out, bool at_noise)
         const size_t m = (size_t) L.maxm;
         const double *Qin = buf[(L.depth + 1) % 2];
         double *Qout = buf[L.depth % 2];
+        if (L.maxm <= DC_SMALL) {
+            k_dc_merge_small<<<L.nnodes, 256, DC_SMALL_SMEM, s>>>(E->nodes, E->pos.lam, E->e, Qin, Qout, n, L.node0, at_noise);
+            g_launches++;
+            g_eig_launches++;
+            continue;
+        }
         k_dc_deflate<<<L.nnodes, 512, 20 * m, s>>>(E->nodes, E->pos, Qin, E->e, n, L.node0);
         k_dc_secular<<<L.nw, 256, 16 * m, s>>>(E->nodes, E->pos, E->tab_w + L.w0, at_noise);
         k_dc_zhat<<<L.nw, 256, 24 * m, s>>>(E->nodes, E->pos, E->tab_w + L.w0);
