@@ -1605,6 +1605,81 @@ __global__ void k_trtri_lower(const double *L, double *Xc, int o)
     }
 }
 
+// The two of them for o up to CQ_MAX with the factor in shared memory (row
+// pitch odd, so a column is read without bank conflicts); every sum keeps its
+// order. k_potrf_small: the kernel above on a resident G. k_trtri_small: a warp
+// per column of the inverse, which adds L(i, k) x(k) to every later i as soon as
+// x(k) is known, instead of a thread per column with a chain of o^2 / 2
+// multiply-adds. o = 161: 473 and 420 us, now 373 and 74 us.
+constexpr int CQ_MAX = 168, CQ_THREADS = 1024;
+__host__ __device__ constexpr int cq_pitch(int o) { return o | 1; }
+size_t cq_smem(int o) { return sizeof(double) * (size_t) o * cq_pitch(o); }
+
+__global__ void __launch_bounds__(CQ_THREADS) k_potrf_small(double *G, int o, int *fail)
+{
+    extern __shared__ double cq[];
+    __shared__ double s_piv;
+    const int ld = cq_pitch(o), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int NW = CQ_THREADS / 32;
+    for (int l = threadIdx.x; l < o * o; l += CQ_THREADS) cq[l / o * ld + l % o] = G[l];
+    __syncthreads();
+    for (int j = 0; j < o; j++) {
+        if (wid == 0) {
+            double s = 0.0;
+            for (int c = lane; c < j; c += 32) s += cq[j * ld + c] * cq[j * ld + c];
+            s = warp_sum_bcast(s);
+            if (lane == 0) {
+                const double ajj = cq[j * ld + j] - s;
+                if (!(ajj > 0.0) || !isfinite(ajj)) *fail = 1;
+                const double l = (ajj > 0.0 && isfinite(ajj)) ? sqrt(ajj) : 1.0;
+                cq[j * ld + j] = l;
+                s_piv = l;
+            }
+        }
+        __syncthreads();
+        const double rinv = 1.0 / s_piv;
+        for (int r = j + 1 + wid; r < o; r += NW) {
+            double s = 0.0;
+            for (int c = lane; c < j; c += 32) s += cq[r * ld + c] * cq[j * ld + c];
+            s = warp_sum_bcast(s);
+            if (lane == 0) cq[r * ld + j] = (cq[r * ld + j] - s) * rinv;
+        }
+        __syncthreads();
+    }
+    for (int l = threadIdx.x; l < o * o; l += CQ_THREADS) G[l] = cq[l / o * ld + l % o];
+}
+
+__global__ void __launch_bounds__(CQ_THREADS) k_trtri_small(const double *L, double *Xc, int o)
+{
+    extern __shared__ double cq[];
+    constexpr int NQ = (CQ_MAX + 31) / 32;
+    const int ld = cq_pitch(o), lane = threadIdx.x & 31, j = blockIdx.x * (CQ_THREADS / 32) + (threadIdx.x >> 5);
+    for (int l = threadIdx.x; l < o * o; l += CQ_THREADS) cq[l / o * ld + l % o] = L[l];
+    __syncthreads();
+    if (j >= o) return;
+    double acc[NQ], x[NQ];   // of rows lane + 32 q
+#pragma unroll
+    for (int q = 0; q < NQ; q++) acc[q] = x[q] = 0.0;
+#pragma unroll
+    for (int kq = 0; kq < NQ; kq++)
+        for (int kl = 0; kl < 32; kl++) {
+            const int k = 32 * kq + kl;
+            if (k < j) continue;
+            if (k >= o) break;
+            const double mine = (k == j ? 1.0 : -acc[kq]) / cq[k * ld + k];
+            if (lane == kl) x[kq] = mine;
+            const double xk = __shfl_sync(0xffffffffu, mine, kl);
+#pragma unroll
+            for (int q = kq; q < NQ; q++) {
+                const int i = lane + 32 * q;
+                if (i > k && i < o) acc[q] = fma(cq[i * ld + k], xk, acc[q]);
+            }
+        }
+#pragma unroll
+    for (int q = 0; q < NQ; q++)
+        if (lane + 32 * q < o) Xc[(size_t) j * o + lane + 32 * q] = x[q];
+}
+
 __global__ void k_hash_fill(double *A, size_t n)
 {
     size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
@@ -1754,7 +1829,7 @@ bool smem_optin()
     if (done_dev == dev) return true;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
     if (!optin_one(k_sytrd_panel, optin) || !optin_one(k_wy_tfactor, optin) || !optin_one(k_dc_deflate, optin) ||
-        !optin_one(k_dc_merge_small, optin) || !optin_one(k_dc_secular, optin) ||
+        !optin_one(k_dc_merge_small, optin) || !optin_one(k_potrf_small, optin) || !optin_one(k_trtri_small, optin) || !optin_one(k_dc_secular, optin) ||
         !optin_one(k_dc_zhat, optin) || !optin_one(k_dc_norms, optin) || !optin_one(k_dc_order, optin))
         return false;
     done_dev = dev;
@@ -1994,8 +2069,13 @@ const int kOrthoEvery = 3;
 void chol_qr(Eig *E, const double *U, double *W, double *G, int n, int o, cudaStream_t s)
 {
     dgemm(false, true, o, o, n, 1.0, U, n, U, n, 0.0, G, o, s);   // G = U U^T
-    k_potrf_lower<<<1, 1024, 0, s>>>(G, o, E->acc);
-    k_trtri_lower<<<(o + 127) / 128, 128, 0, s>>>(G, E->Gx, o);
+    if (o <= CQ_MAX) {
+        k_potrf_small<<<1, CQ_THREADS, cq_smem(o), s>>>(G, o, E->acc);
+        k_trtri_small<<<(o + CQ_THREADS / 32 - 1) / (CQ_THREADS / 32), CQ_THREADS, cq_smem(o), s>>>(G, E->Gx, o);
+    } else {
+        k_potrf_lower<<<1, 1024, 0, s>>>(G, o, E->acc);
+        k_trtri_lower<<<(o + 127) / 128, 128, 0, s>>>(G, E->Gx, o);
+    }
     g_launches += 2;
     // row-major Gx is (L^-1)^T, so W = Gx^T U
     dgemm(true, false, o, n, o, 1.0, E->Gx, o, U, n, 0.0, W, n, s);
