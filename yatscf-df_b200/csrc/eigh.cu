@@ -1905,6 +1905,8 @@ void eig_destroy(Eig *e)
     delete e;
 }
 
+bool eig_small_launches(const Eig *e) { return e->cluster && trc_in_smem(e->n, e->n); }
+
 int eig_error(Eig *e)
 {
     int v = 0;

@@ -16,10 +16,9 @@
 // of libCMS/CMS_Simint.c:131-141 does.
 #include <cmath>
 #include <cstdio>
-#include <map>
-#include <mutex>
 #include <vector>
 
+#include "fork.h"
 #include "ints_unrolled.cuh"
 #include "tscf_internal.h"
 #include "tune.h"
@@ -96,93 +95,10 @@ __device__ __forceinline__ Sh load_shell(const DevShells &s, int i)
     return r;
 }
 
-// ------------------------------------------------------------------ class launches side by side
-// The angular-momentum classes of one integral kind write disjoint outputs, and
-// a small molecule's classes are a few blocks each whose threads run their
-// primitives as a serial chain (0.1 to 1.4 ms per class on water): one after
-// another on one stream they leave the chip idle. A Fork runs them on LANES
-// streams between an event on the caller's stream and events that it waits for.
-// Streams and events come from a per-device pool of at most KEEP sets (a set
-// belongs to one Fork at a time), so nothing is created per call.
-class Fork {
-    static constexpr int LANES = 8, KEEP = 4;
-    struct Set {
-        cudaStream_t st[LANES] = {};
-        cudaEvent_t begin = nullptr, done[LANES] = {};
-        bool ok = true;
-        Set()
-        {
-            ok = cudaEventCreateWithFlags(&begin, cudaEventDisableTiming) == cudaSuccess;
-            for (int k = 0; k < LANES; k++)
-                ok = ok && cudaStreamCreateWithFlags(&st[k], cudaStreamNonBlocking) == cudaSuccess &&
-                     cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming) == cudaSuccess;
-        }
-        ~Set()
-        {
-            for (int k = 0; k < LANES; k++) {
-                if (st[k]) cudaStreamDestroy(st[k]);
-                if (done[k]) cudaEventDestroy(done[k]);
-            }
-            if (begin) cudaEventDestroy(begin);
-        }
-    };
-    static std::mutex &lock()
-    {
-        static std::mutex *m = new std::mutex;
-        return *m;
-    }
-    static std::vector<Set *> &pool(int dev)
-    {
-        static auto *p = new std::map<int, std::vector<Set *>>;   // outlives static destruction
-        return (*p)[dev];
-    }
-    int dev_ = 0, n_ = 0;
-    cudaStream_t s_;
-    Set *set_ = nullptr;
-
-public:
-    // side = false: every launch stays on s
-    Fork(cudaStream_t s, bool side) : s_(s)
-    {
-        if (!side) return;
-        cudaGetDevice(&dev_);
-        {
-            std::lock_guard<std::mutex> g(lock());
-            auto &v = pool(dev_);
-            if (!v.empty()) {
-                set_ = v.back();
-                v.pop_back();
-            }
-        }
-        if (!set_) set_ = new Set;
-        if (!set_->ok || cudaEventRecord(set_->begin, s) != cudaSuccess) {
-            cudaGetLastError();
-            delete set_;
-            set_ = nullptr;
-        }
-    }
-    Fork(const Fork &) = delete;
-    Fork &operator=(const Fork &) = delete;
-    cudaStream_t next()
-    {
-        if (!set_) return s_;
-        const int k = n_++ % LANES;
-        if (n_ <= LANES) cudaStreamWaitEvent(set_->st[k], set_->begin, 0);
-        return set_->st[k];
-    }
-    ~Fork()
-    {
-        if (!set_) return;
-        for (int k = 0; k < LANES && k < n_; k++) {
-            cudaEventRecord(set_->done[k], set_->st[k]);
-            cudaStreamWaitEvent(s_, set_->done[k], 0);
-        }
-        std::lock_guard<std::mutex> g(lock());
-        auto &v = pool(dev_);
-        if ((int) v.size() < KEEP) v.push_back(set_);
-        else delete set_;
-    }
-};
+// The angular-momentum classes of one integral kind write disjoint outputs, and a
+// small molecule's classes are a few blocks each whose threads run their primitives
+// as a serial chain (0.1 to 1.4 ms per class on water): they are launched side by
+// side (Fork), not one after another.
 
 // ------------------------------------------------------------------ primitive quartets, unrolled
 constexpr double TWO_PI_52 = 2.0 * 17.493418327624862;   // 2 pi^2.5

@@ -7,11 +7,13 @@
 #include <cstdio>
 #include <cstdint>
 #include <cstdlib>
+#include <map>
 #include <mutex>
 
 #include <utility>
 #include <vector>
 
+#include "fork.h"
 #include "tiles.cuh"
 #include "tune.h"
 #include "tscf_internal.h"
@@ -19,6 +21,18 @@
 namespace tscf {
 
 std::atomic<long long> g_launches{0};
+
+// the pools of fork.h outlive static destruction
+std::mutex &Fork::lock()
+{
+    static std::mutex *m = new std::mutex;
+    return *m;
+}
+std::vector<Fork::Set *> &Fork::pool(int dev)
+{
+    static auto *p = new std::map<int, std::vector<Set *>>;
+    return (*p)[dev];
+}
 
 // ------------------------------------------------------------------ DGEMM
 // Five tile shapes: FFMA 64x64 (default), 32x32 (more blocks for small

@@ -450,7 +450,7 @@ static void inv_sqrt_ns(const double *M, double *Y, double *Z, double *T, double
 }
 
 // res = max|R|, R = (I - U^T U) F' U^T; UA = U F' U^T
-static void refine_residual(const double *d_Fp, const double *d_U, int n, int o, SubspaceWork &w, cudaStream_t s)
+void subspace_residual(const double *d_Fp, const double *d_U, int n, int o, SubspaceWork &w, cudaStream_t s)
 {
     dgemm(false, true, n, o, n, 1.0, d_Fp, n, d_U, n, 0.0, w.A, o, s);          // A = F' U^T (n x o)
     dgemm(false, false, o, o, n, 1.0, d_U, n, w.A, o, 0.0, w.UA, o, s);        // UA = U F' U^T
@@ -462,8 +462,8 @@ static void refine_residual(const double *d_Fp, const double *d_U, int n, int o,
 }
 
 // one preconditioned step on U followed by Loewdin re-orthonormalisation
-static void refine_update(const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o, SubspaceWork &w,
-                          cudaStream_t s)
+void subspace_update(const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o, SubspaceWork &w,
+                     cudaStream_t s)
 {
     const int v = n - o;
     const double *Vv = d_Vstale + (size_t) o * n;
@@ -489,18 +489,23 @@ __host__ __device__ inline bool refine_continue(double res, double prev, int ste
     return res * pow(res / prev, max_steps - step) <= tol;
 }
 
+bool subspace_continue(double res, double prev, int step, int max_steps, double tol)
+{
+    return refine_continue(res, prev, step, max_steps, tol);
+}
+
 int subspace_refine(const double *d_Fp, const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o,
                     SubspaceWork &w, double tol, int max_steps, int *steps_out, double *res_out, cudaStream_t s)
 {
     double res = 1e300, prev = 1e300;
     int step = 0;
     for (;; step++) {
-        refine_residual(d_Fp, d_U, n, o, w, s);
+        subspace_residual(d_Fp, d_U, n, o, w, s);
         cudaMemcpyAsync(&res, w.res, sizeof(double), cudaMemcpyDeviceToHost, s);
         if (cudaStreamSynchronize(s) != cudaSuccess) return ERR_CUDA;
         if (!refine_continue(res, prev, step, max_steps, tol)) break;
         prev = res;
-        refine_update(d_Vstale, d_wstale, d_U, n, o, w, s);
+        subspace_update(d_Vstale, d_wstale, d_U, n, o, w, s);
     }
     *steps_out = step;
     *res_out = res;
@@ -529,7 +534,7 @@ int subspace_refine_capture(const double *d_Fp, const double *d_Vstale, const do
                             int o, SubspaceWork &w, RefineCtl *d_ctl, cudaStream_t s, cudaStream_t s_body,
                             long long *body_launches)
 {
-    refine_residual(d_Fp, d_U, n, o, w, s);
+    subspace_residual(d_Fp, d_U, n, o, w, s);
     cudaStreamCaptureStatus st;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t *deps = nullptr;
@@ -554,8 +559,8 @@ int subspace_refine_capture(const double *d_Fp, const double *d_Vstale, const do
     if (cudaStreamBeginCaptureToGraph(s_body, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)
         return ERR_CUDA;
     const long long l0 = g_launches;
-    refine_update(d_Vstale, d_wstale, d_U, n, o, w, s_body);
-    refine_residual(d_Fp, d_U, n, o, w, s_body);
+    subspace_update(d_Vstale, d_wstale, d_U, n, o, w, s_body);
+    subspace_residual(d_Fp, d_U, n, o, w, s_body);
     k_refine_decide<<<1, 1, 0, s_body>>>(d_ctl, w.res, h, 0);
     g_launches++;
     *body_launches = g_launches - l0;

@@ -154,6 +154,8 @@ void eig_destroy(Eig *e);
 // at_noise: the secular equation's roots stop where its value is rounding (k_dc_secular).
 int  eig_run(Eig *e, const double *d_A, double *d_w, double *d_V, cudaStream_t s, bool at_noise = false);
 int  eig_error(Eig *e);
+// Whether every panel runs as one cluster (no cooperative launch that needs all the chip).
+bool eig_small_launches(const Eig *e);
 
 // Orthonormal rows U (o x n) spanning the dominant o-dimensional invariant
 // subspace of a symmetric M (n x n): iters products with M from a fixed
@@ -293,6 +295,10 @@ struct SubspaceWork {
 };
 int subspace_refine(const double *d_Fp, const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o,
                     SubspaceWork &w, double tol, int max_steps, int *steps_out, double *res_out, cudaStream_t s);
+void subspace_residual(const double *d_Fp, const double *d_U, int n, int o, SubspaceWork &w, cudaStream_t s);   // into w.res
+void subspace_update(const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o, SubspaceWork &w,
+                     cudaStream_t s);
+bool subspace_continue(double res, double prev, int step, int max_steps, double tol);
 // Refinement inside a stream capture: the steps run in a WHILE conditional
 // node whose condition a device kernel sets from the residual. d_ctl->tol and
 // ->max_steps are inputs; ->step, ->res and ->converged are written.
