@@ -17,6 +17,7 @@
 #include "tiles.cuh"
 #include "tune.h"
 #include "tscf_internal.h"
+#include "umma.cuh"
 
 namespace tscf {
 
@@ -67,15 +68,187 @@ __global__ void __launch_bounds__(256, 1) k_dgemm_dmma(int m, int n, int k, doub
     dgemm_tile_dmma<TA, TB>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, blockIdx.y * 128, blockIdx.x * 128);
 }
 
+static bool dgemm_bulk_fits(bool ta, bool tb, int m, int n, int k, const double *A, int lda, const double *B, int ldb,
+                            double beta, const double *C, int ldc);
+static bool dgemm_bulk(int m, int n, int k, double alpha, const double *A, int lda, const double *B, int ldb, double *C,
+                       int ldc, cudaStream_t s);
+
 static void dgemm_dmma(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda, const double *B,
                        int ldb, double beta, double *C, int ldc, cudaStream_t s)
 {
+    if (dgemm_bulk_fits(ta, tb, m, n, k, A, lda, B, ldb, beta, C, ldc) && dgemm_bulk(m, n, k, alpha, A, lda, B, ldb, C, ldc, s))
+        return;
     dim3 grid((n + 127) / 128, (m + 127) / 128);
     g_launches++;
     if (!ta && !tb) k_dgemm_dmma<false, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
     else if (!ta && tb) k_dgemm_dmma<false, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
     else if (ta && !tb) k_dgemm_dmma<true, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
     else k_dgemm_dmma<true, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+
+// ---- the same product for large A B with row-major operands in whole 16-byte
+// units: 168 x 96 tiles over 12 warps of 56 x 24 in a persistent CTA per SM,
+// fed by a producer warp (the fourth warp of one SM quarter, which leaves each
+// 128 registers). Lane 0 of it loads 32-wide K chunks by TMA, two chunks ahead,
+// behind mbarriers, so the other warps issue nothing but fragment reads and
+// DMMAs and never wait for one another. Neighbouring CTAs take the tiles of one
+// row block, so A comes from HBM once and B stays in L2. Each output is one FMA
+// chain over k, as in every other tile but the K-split one: the same bits.
+// DMMA rate bounds it: C40H82's DF tensor (122,420 x 3870 x 3870) takes 105 ms,
+// 34.9 TF/s or 94% of that rate, against 133 ms on the 128 x 128 tile above. With
+// one untiled bulk copy per row (256 B of A, 768 B of B) instead of tensor boxes
+// it took 145 ms.
+// Shared memory: boxes of 16 doubles (128 B) a row in the 128-byte swizzle, two of
+// 168 rows of A, six of 32 rows of B. Fragment row fr is tile row perm(fr), and
+// fragment column fr is column colperm(fr) of a 16-column box, such that the 16
+// lanes of a half-warp read 16 different bank pairs.
+constexpr int BG_WM = 3, BG_NX = 7, BG_WN = 4, BG_NY = 3;
+constexpr int BG_M = BG_WM * BG_NX * 8, BG_N = BG_WN * BG_NY * 8, BG_K = 32;
+constexpr int BG_WARPS = BG_WM * BG_WN, BG_THREADS = (BG_WARPS + 1) * 32, BG_STAGES = 3;
+constexpr int BG_ABOX = BG_M * 16, BG_BBOX = BG_K * 16;   // doubles
+constexpr int BG_STAGE = BG_K / 16 * BG_ABOX + BG_N / 16 * BG_BBOX;
+constexpr size_t BG_SMEM = sizeof(double) * BG_STAGES * BG_STAGE + 1024;
+constexpr long long BG_WAIT = 2000000000LL;   // clock cycles a barrier wait may take (~1 s)
+static_assert(BG_SMEM + 64 <= 227 * 1024 && BG_M <= 256, "bulk GEMM stages exceed shared memory");
+static_assert(BG_ABOX % 128 == 0 && BG_BBOX % 128 == 0, "swizzled boxes start at multiples of 1024 bytes");
+__device__ int g_gemm_error;
+
+__global__ void __launch_bounds__(BG_THREADS, 1)
+    k_dgemm_bulk(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, int m, int n, int k,
+                 double alpha, double *__restrict__ C, int ldc, int ntn, int ntiles)
+{
+    extern __shared__ __align__(1024) unsigned char bg_raw[];
+    double *bgsm = (double *) (((uintptr_t) bg_raw + 1023) & ~(uintptr_t) 1023);
+    __shared__ uint64_t full[BG_STAGES], empty[BG_STAGES];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        for (int q = 0; q < BG_STAGES; q++) {
+            umma::mbar_init(&full[q], 1);
+            umma::mbar_init(&empty[q], BG_WARPS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async;" ::: "memory");
+    }
+    __syncthreads();
+    int st = 0, phase = 0;
+    if (warp == BG_WARPS) {   // ---- producer
+        if (lane != 0) return;
+        bool first = true;    // the first BG_STAGES chunks find their stage empty
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            const int m0 = t / ntn * BG_M, n0 = t % ntn * BG_N;
+            for (int k0 = 0; k0 < k; k0 += BG_K) {
+                if (!first && !umma::mbar_wait_bounded(&empty[st], phase ^ 1, &g_gemm_error, 41, BG_WAIT)) {
+                    for (int q = 0; q < BG_STAGES; q++) {   // its copies in flight, oldest first
+                        umma::mbar_wait_bounded(&full[st], phase ^ 1, &g_gemm_error, 42, BG_WAIT);
+                        if (++st == BG_STAGES) {
+                            st = 0;
+                            phase ^= 1;
+                        }
+                    }
+                    return;
+                }
+                double *As = bgsm + (size_t) st * BG_STAGE, *Bs = As + BG_K / 16 * BG_ABOX;
+                umma::mbar_expect_tx(&full[st], (unsigned) (sizeof(double) * BG_STAGE));
+#pragma unroll
+                for (int q = 0; q < BG_K / 16; q++) umma::tma_load_2d(As + q * BG_ABOX, &mA, &full[st], k0 + 16 * q, m0);
+#pragma unroll
+                for (int q = 0; q < BG_N / 16; q++) umma::tma_load_2d(Bs + q * BG_BBOX, &mB, &full[st], n0 + 16 * q, k0);
+                if (++st == BG_STAGES) {
+                    st = 0;
+                    phase ^= 1;
+                    first = false;
+                }
+            }
+        }
+        return;
+    }
+    const int wm = (warp / BG_WN) * BG_NX * 8, f0 = (warp % BG_WN) * BG_NY;   // f0: first 8-column fragment
+    const int fr = lane >> 2, fc = lane & 3, perm = (2 * fr & 7) | (fr >> 2);
+    // element (r, kk) of A's box: 16 r + 2 ((kk / 2) ^ (r & 7)) + kk % 2; B's (kk, c) alike
+    const int oa = (wm + perm) * 16 + (((fc >> 1) ^ perm) << 1) + (fc & 1);
+    int ob[BG_NY];
+#pragma unroll
+    for (int y = 0; y < BG_NY; y++) {
+        const int f = f0 + y, chunk = ((f & 1) << 1) | ((fr & 2) << 1) | (fr >> 2);
+        ob[y] = (f >> 1) * BG_BBOX + fc * 16 + ((chunk ^ fc) << 1) + (fr & 1);
+    }
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int m0 = t / ntn * BG_M, n0 = t % ntn * BG_N;
+        double acc[BG_NX][BG_NY][2];
+#pragma unroll
+        for (int x = 0; x < BG_NX; x++)
+#pragma unroll
+            for (int y = 0; y < BG_NY; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
+        for (int k0 = 0; k0 < k; k0 += BG_K) {
+            if (!umma::mbar_wait_bounded(&full[st], phase, &g_gemm_error, 43, BG_WAIT)) return;
+            const double *As = bgsm + (size_t) st * BG_STAGE, *Bs = As + BG_K / 16 * BG_ABOX;
+#pragma unroll
+            for (int k4 = 0; k4 < BG_K; k4 += 4) {   // zeros behind k, m and n
+                double a[BG_NX], b[BG_NY];
+                const double *ap = As + k4 / 16 * BG_ABOX + (oa ^ (k4 % 16));
+#pragma unroll
+                for (int x = 0; x < BG_NX; x++) a[x] = ap[128 * x];
+#pragma unroll
+                for (int y = 0; y < BG_NY; y++) b[y] = Bs[(ob[y] ^ (2 * (k4 & 4))) + 16 * k4];
+#pragma unroll
+                for (int x = 0; x < BG_NX; x++)
+#pragma unroll
+                    for (int y = 0; y < BG_NY; y++) dmma_8x8x4(acc[x][y][0], acc[x][y][1], a[x], b[y]);
+            }
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&empty[st]);
+            if (++st == BG_STAGES) {
+                st = 0;
+                phase ^= 1;
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < BG_NX; x++) {
+            const int gi = m0 + wm + 8 * x + perm;
+#pragma unroll
+            for (int y = 0; y < BG_NY; y++) {
+                const int f = f0 + y, gj = n0 + (f >> 1) * 16 + 4 * (f & 1) + 8 * (fc & 1) + 2 * (fc >> 1);
+                if (gi < m && gj < n)
+                    *reinterpret_cast<double2 *>(C + (size_t) gi * ldc + gj) =
+                        make_double2(alpha * acc[x][y][0], alpha * acc[x][y][1]);
+            }
+        }
+    }
+}
+
+// Whether k_dgemm_bulk takes the product: 16-byte units throughout, C written
+// only, and enough tiles that the last wave costs little.
+static bool dgemm_bulk_fits(bool ta, bool tb, int m, int n, int k, const double *A, int lda, const double *B, int ldb,
+                            double beta, const double *C, int ldc)
+{
+    if (ta || tb || beta != 0.0 || k < BG_K || ((lda | ldb | ldc | n | k) & 1)) return false;
+    if (((uintptr_t) A | (uintptr_t) B | (uintptr_t) C) & 15) return false;
+    const long long tiles = (long long) ((m + BG_M - 1) / BG_M) * ((n + BG_N - 1) / BG_N);
+    return tiles >= 4LL * num_sms() && tiles < (1LL << 31);
+}
+
+static bool dgemm_bulk(int m, int n, int k, double alpha, const double *A, int lda, const double *B, int ldb, double *C,
+                       int ldc, cudaStream_t s)
+{
+    CUtensorMap mA, mB;
+    if (!umma::make_map_2d(&mA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, m, k, lda, 16, BG_M) ||
+        !umma::make_map_2d(&mB, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, B, k, n, ldb, 16, BG_K))
+        return false;
+    if (cudaFuncSetAttribute(k_dgemm_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) BG_SMEM) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const int ntn = (n + BG_N - 1) / BG_N, ntiles = ntn * ((m + BG_M - 1) / BG_M);
+    k_dgemm_bulk<<<num_sms(), BG_THREADS, BG_SMEM, s>>>(mA, mB, m, n, k, alpha, C, ldc, ntn, ntiles);
+    g_launches++;
+    return true;
+}
+
+int gemm_error_flag()
+{
+    int v = 0;
+    cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(int));
+    return v;
 }
 
 template <bool TA, bool TB>

@@ -1261,6 +1261,10 @@ int df_impl(TinySCF_t t)
     tstop(e, TINYSCF_T_DFGEMM);
     RC(cuda_rc("DF tensor GEMM"));
     int rc = sync_rc(e, "DF tensor");
+    if (const int fl = rc ? 0 : gemm_error_flag()) {
+        fprintf(stderr, "[tinyscf] DF tensor GEMM: a bounded wait timed out (code %d)\n", fl);
+        rc = ERR_CUDA;
+    }
     eig_destroy(eg);
     dfree(e, pqA);
     dfree(e, Jpq);
@@ -1687,6 +1691,10 @@ int scf_impl(TinySCF_t t)
     }
     if (const int fl = half_error_flag()) {
         fprintf(stderr, "[tinyscf] exchange half-transform: a bounded wait timed out (code %d)\n", fl);
+        return ERR_CUDA;
+    }
+    if (const int fl = gemm_error_flag()) {
+        fprintf(stderr, "[tinyscf] FP64 GEMM: a bounded wait timed out (code %d)\n", fl);
         return ERR_CUDA;
     }
     if (e->oz) {

@@ -120,6 +120,7 @@ int device_bf_fill(const double *d_bf_scr, int n, double eta, const int *d_work,
 void dgemm(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda,
            const double *B, int ldb, double beta, double *C, int ldc, cudaStream_t s);
 
+int gemm_error_flag();   // nonzero: a bounded wait of k_dgemm_bulk gave up
 // The same product with the tile picked from the call shape (no tuning run).
 void dgemm_untuned(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda,
                    const double *B, int ldb, double beta, double *C, int ldc, cudaStream_t s);
