@@ -211,6 +211,20 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_sytrd_panel(TrdArgs a)
         }
         ss = block_sum_all<TRD_THREADS>(ss, s_red);
         if (tid == 0) part_n[blockIdx.x] = ss;
+        // items (row rr, segment sg) of phase 2's y = A v, over rows j+1..n-1 and the segments holding
+        // columns j+1..n-1; A does not change within the panel, so a warp's first item is loaded here
+        const int s0 = (j + 1) / TRD_SEG, ns = nseg - s0, nitems = (n - j - 1) * ns;
+        double av[TRD_SEG / 32];
+        auto load_item = [&](int it) {
+            const int rr = j + 1 + it / ns, sg = s0 + it % ns;
+            const double *row = A + (size_t) rr * n + sg * TRD_SEG + lane;
+#pragma unroll
+            for (int k = 0; k < TRD_SEG / 32; k++) {
+                const int c2 = sg * TRD_SEG + lane + 32 * k;
+                av[k] = (it < nitems && c2 > j && c2 < n) ? row[32 * k] : 0.0;
+            }
+        };
+        if (j < n - 1) load_item(gw);
         if (!grid_barrier(a.bar, a.err, a.G)) return;
         if (j == n - 1) {
             if (gtid == 0) a.d[j] = a.col[j];
@@ -259,18 +273,18 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_sytrd_panel(TrdArgs a)
                 if (q == (c >> 3)) pv[q] = vr_own;
         }
         {
-            // items (row rr, segment sg) over rows j+1..n-1 and the segments holding columns j+1..n-1
-            const int s0 = (j + 1) / TRD_SEG, ns = nseg - s0, m = n - j - 1;
-            const long long nitems = (long long) m * ns;
-            for (long long it = gw; it < nitems; it += GW) {
-                const int rr = j + 1 + (int) (it / ns), sg = s0 + (int) (it % ns);
-                const double *row = A + (size_t) rr * n;
+            // the next item's loads are issued before this one's sum, which is a chain of shuffles: at n = 3870
+            // (26 items a warp in the first columns) the panels took 85 ms without, now 72 ms; 4.7 ms of the panels
+            // above 600 rows at n = 1010 (1 or 2 items) did not change
+            for (int it = gw; it < nitems; it += GW) {
+                const int rr = j + 1 + it / ns, sg = s0 + it % ns;
                 double acc[TRD_SEG / 32];
 #pragma unroll
                 for (int k = 0; k < TRD_SEG / 32; k++) {
                     const int c2 = sg * TRD_SEG + lane + 32 * k;
-                    acc[k] = (c2 > j && c2 < n) ? row[c2] * sv[c2] : 0.0;
+                    acc[k] = (c2 > j && c2 < n) ? av[k] * sv[c2] : 0.0;
                 }
+                load_item(it + GW);
                 static_assert(TRD_SEG == 256, "the pairwise sum below is written for 8 values per lane");
                 const double y = warp_sum_bcast(((acc[0] + acc[4]) + (acc[2] + acc[6])) +
                                                 ((acc[1] + acc[5]) + (acc[3] + acc[7])));
@@ -307,7 +321,6 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_sytrd_panel(TrdArgs a)
         if (!grid_barrier(a.bar, a.err, a.G)) return;
         // ---- phase 3: w = tau (y - V (W^T v) - W (V^T v)) for this row, partial w.v
         double ypart = 0.0;
-        const int s0 = (j + 1) / TRD_SEG;
         if (own && r > j)
             for (int sg = s0 + l8; sg < nseg; sg += 8) ypart += a.y[(size_t) sg * n + r];
         for (int cc = wid; cc < c; cc += TRD_THREADS / 32) {
