@@ -217,14 +217,22 @@ __global__ void __launch_bounds__(BG_THREADS, 1)
 }
 
 // Whether k_dgemm_bulk takes the product: 16-byte units throughout, C written
-// only, and enough tiles that the last wave costs little.
+// only, and its waves of 168 x 96 tiles at 94% of the DMMA rate cost less than
+// those of 128 x 128 tiles at 75%. Measured, bulk against 128 x 128 (ms):
+// 1010^3 0.144 / 0.186, 1680^3 0.460 / 0.588, 1950^3 0.526 / 0.685, 3072^3
+// 2.04 / 2.12, 3870^3 3.58 / 4.66, 33600 x 960 x 960 1.81 / 2.52, 3870 x 3870 x 64
+// 0.087 / 0.127; where its last wave is nearly empty (2688^3, 3.03 waves)
+// 1.43 / 1.40, which the rule leaves to the 128 x 128 tile.
 static bool dgemm_bulk_fits(bool ta, bool tb, int m, int n, int k, const double *A, int lda, const double *B, int ldb,
                             double beta, const double *C, int ldc)
 {
     if (ta || tb || beta != 0.0 || k < BG_K || ((lda | ldb | ldc | n | k) & 1)) return false;
     if (((uintptr_t) A | (uintptr_t) B | (uintptr_t) C) & 15) return false;
+    const long long nsm = num_sms();
     const long long tiles = (long long) ((m + BG_M - 1) / BG_M) * ((n + BG_N - 1) / BG_N);
-    return tiles >= 4LL * num_sms() && tiles < (1LL << 31);
+    const long long old = (long long) ((m + 127) / 128) * ((n + 127) / 128);
+    const double waves = (double) ((tiles + nsm - 1) / nsm), old_waves = (double) ((old + nsm - 1) / nsm);
+    return tiles < (1LL << 31) && waves * (BG_M * BG_N) / 0.94 < old_waves * (128 * 128) / 0.75;
 }
 
 static bool dgemm_bulk(int m, int n, int k, double alpha, const double *A, int lda, const double *B, int ldb, double *C,
@@ -239,7 +247,7 @@ static bool dgemm_bulk(int m, int n, int k, double alpha, const double *A, int l
         return false;
     }
     const int ntn = (n + BG_N - 1) / BG_N, ntiles = ntn * ((m + BG_M - 1) / BG_M);
-    k_dgemm_bulk<<<num_sms(), BG_THREADS, BG_SMEM, s>>>(mA, mB, m, n, k, alpha, C, ldc, ntn, ntiles);
+    k_dgemm_bulk<<<std::min(ntiles, num_sms()), BG_THREADS, BG_SMEM, s>>>(mA, mB, m, n, k, alpha, C, ldc, ntn, ntiles);
     g_launches++;
     return true;
 }
