@@ -760,6 +760,7 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) k_sytrd_cluster(TrdArgs a)
                 if (q == (c >> 3)) pw[q] += a2 * pv[q];
         }
     }
+    __syncthreads();   // s_d of the last column: written by thread 0, read below by the column's own thread
     // the reflectors, and the final W of the rows behind the panel, into both stacked panels (nothing is written
     // to global memory inside the loop: a barrier's release would wait for it)
     if (own) {
