@@ -275,6 +275,12 @@ TINYSCF_API int TinySCF_set_JK(TinySCF_t t, const double *J, const double *K);
  * memory and returns. *code receives that code (0 if no wait gave up); the
  * flag is cleared afterwards and the handle stays usable. */
 TINYSCF_API int TinySCF_kmix_wait_probe(TinySCF_t t, long long wait_cycles, int *code);
+/* Every wait inside the engine's kernels is bounded; a kernel that gives up
+ * leaves its output incomplete, and the call that waits for it, or the next one
+ * on any handle, returns TINYSCF_ERR_CUDA. The report clears the condition.
+ * This runs one wait of wait_cycles clock cycles out on a barrier that nothing
+ * completes and leaves it unreported, to check the reports. */
+TINYSCF_API int TinySCF_wait_probe(TinySCF_t t, long long wait_cycles);
 /* The engine's FP64 symmetric eigensolver on host buffers: A (n x n,
  * row-major, symmetric) -> w (n eigenvalues, ascending) and V (n x n, row k =
  * eigenvector k). It is what replaces the reference's LAPACKE_dsyev calls

@@ -21,7 +21,7 @@
 //     (H_p..H_(p+nb-1) = I - V T V^T), three GEMMs per panel.
 //
 // Every grid barrier spins a bounded number of times; a barrier that runs out
-// sets the object's error flag and every CTA returns (eig_error() reports it).
+// sets the process's wait word (waits_check reports it) and every CTA returns.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -135,7 +135,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long *bar, int *err, 
         bool ok = true;
         while (ld_acquire(bar) < target) {
             if (++spins > kBarrierSpins) {
-                atomicExch(err, 1);
+                *(volatile int *) err = 51;
                 ok = false;
                 break;
             }
@@ -1715,7 +1715,6 @@ struct Eig {
     double *A = nullptr, *VT = nullptr, *PVW = nullptr, *PWV = nullptr, *d = nullptr, *e = nullptr, *tau = nullptr,
            *col = nullptr, *y = nullptr, *part = nullptr, *Gb = nullptr, *Tf = nullptr, *Y = nullptr, *Y2 = nullptr;
     unsigned long long *bar = nullptr;
-    int *err = nullptr;
     // divide and conquer: eigenvector buffers of alternate tree levels (Qa reuses A) and the merge's U
     double *Qb = nullptr, *Us = nullptr;
     DcNodes nodes{};
@@ -1886,7 +1885,7 @@ Eig *eig_create(int n, cudaStream_t s)
               ealloc(E, &E->part, (size_t) E->G * (2 + 2 * TRD_NB)) &&
               ealloc(E, &E->Gb, (size_t) std::max(E->nblk, 1) * GR_KS * BT_NB * BT_NB) &&
               ealloc(E, &E->Tf, (size_t) std::max(E->nblk, 1) * BT_NB * BT_NB) && ealloc(E, &E->bar, 2) &&
-              ealloc(E, &E->err, 1) && ealloc(E, &E->acc, 1);
+              ealloc(E, &E->acc, 1) && wait_word() != nullptr;
     DcPos &P = E->pos;
     ok = ok && ealloc(E, &P.lam, n) && ealloc(E, &P.ds, n) && ealloc(E, &P.dK, n) && ealloc(E, &P.zK, n) &&
          ealloc(E, &P.lamb, n) && ealloc(E, &P.tau, n) && ealloc(E, &P.zh, n) && ealloc(E, &P.nrm, n) &&
@@ -1901,7 +1900,6 @@ Eig *eig_create(int n, cudaStream_t s)
     cudaMemset(P.colsrc, 0, sizeof(int) * n);
     cudaMemset(P.perm, 0, sizeof(int) * n);
     cudaMemset(E->bar, 0, sizeof(unsigned long long));
-    cudaMemset(E->err, 0, sizeof(int));
     const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) {
         fprintf(stderr, "[tinyscf] eigensolver set-up for n = %d: %s\n", n, cudaGetErrorString(err));
@@ -1920,14 +1918,6 @@ void eig_destroy(Eig *e)
 }
 
 bool eig_small_launches(const Eig *e) { return e->cluster && trc_in_smem(e->n, e->n); }
-
-int eig_error(Eig *e)
-{
-    int v = 0;
-    if (!e) return ERR_STATE;
-    if (cudaMemcpy(&v, e->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return ERR_CUDA;
-    return v ? ERR_CUDA : OK;
-}
 
 namespace {
 
@@ -1954,7 +1944,7 @@ int tridiagonalize(Eig *E, const double *d_A, cudaStream_t s)
         a.y = E->y;
         a.part = E->part;
         a.bar = E->bar;
-        a.err = E->err;
+        a.err = wait_word();
         a.n = n;
         a.p = P * TRD_NB;
         a.cols = std::min(TRD_NB, n - a.p);

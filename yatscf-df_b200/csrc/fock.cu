@@ -357,7 +357,6 @@ __global__ void __launch_bounds__(KhTile<WS, NX, WP, NY>::THREADS, 1)
 // that holds the producer as its fourth warp gives each 128 registers, which
 // bounds the tile of 12 warps (56 x 24 a warp).
 constexpr long long KH_WAIT = 2000000000LL;   // clock cycles a barrier wait may take (~1 s)
-__device__ int g_half_error;
 
 __device__ __forceinline__ void bulk_row(double *dst, const double *src, unsigned bytes, uint64_t *bar)
 {
@@ -390,7 +389,7 @@ __global__ void __launch_bounds__(KhBulk<WS, NX, WP, NY>::THREADS, 1)
     k_halftransform_bulk(const double *__restrict__ B, const double *__restrict__ Cp, int cp, const double *zeros,
                          const int *__restrict__ csr_j, const int *__restrict__ csr_u, const int *__restrict__ displs,
                          int nocc, int naux, double *__restrict__ T, int n_items, int stiles, int ptiles,
-                         unsigned long long *rowmax)
+                         unsigned long long *rowmax, int *gave_up)
 {
     using K = KhBulk<WS, NX, WP, NY>;
     constexpr int S = K::S, PW = K::P, ST = K::STAGES;
@@ -419,9 +418,9 @@ __global__ void __launch_bounds__(KhBulk<WS, NX, WP, NY>::THREADS, 1)
         fetch();
         for (int g = 0; Q.item < n_items; g++) {
             const int st = g % ST;
-            if (g >= ST && !umma::mbar_wait_bounded(&empty[st], ((g / ST) - 1) & 1, &g_half_error, 31, KH_WAIT)) {
+            if (g >= ST && !umma::mbar_wait_bounded(&empty[st], ((g / ST) - 1) & 1, gave_up, 31, KH_WAIT)) {
                 for (int k = g - ST; k < g; k++)   // its copies in flight
-                    umma::mbar_wait_bounded(&full[k % ST], (k / ST) & 1, &g_half_error, 32, KH_WAIT);
+                    umma::mbar_wait_bounded(&full[k % ST], (k / ST) & 1, gave_up, 32, KH_WAIT);
                 return;
             }
             double *As = khsm + (size_t) st * K::STAGE, *Bs = As + KT_K * K::AS;
@@ -444,7 +443,7 @@ __global__ void __launch_bounds__(KhBulk<WS, NX, WP, NY>::THREADS, 1)
         for (int y = 0; y < NY; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
     int st = 0, phase = 0;
     while (Q.item < n_items) {
-        if (!umma::mbar_wait_bounded(&full[st], phase, &g_half_error, 33, KH_WAIT)) return;
+        if (!umma::mbar_wait_bounded(&full[st], phase, gave_up, 33, KH_WAIT)) return;
         const double *As = khsm + (size_t) st * K::STAGE + fc * K::AS + ws + fr;
         const double *Bs = khsm + (size_t) st * K::STAGE + KT_K * K::AS + fc * K::BS + wp + fr;
 #pragma unroll
@@ -489,13 +488,6 @@ __global__ void __launch_bounds__(KhBulk<WS, NX, WP, NY>::THREADS, 1)
     }
 }
 
-int half_error_flag()
-{
-    int v = 0;
-    cudaMemcpyFromSymbol(&v, g_half_error, sizeof(int));
-    return v;
-}
-
 // Doubles of FockPlan::Cpad for nbf x nocc: rows padded to whole tiles, and a block of zeros.
 size_t half_pad_elems(int nbf, int nocc)
 {
@@ -516,7 +508,7 @@ static void launch_half(const FockPlan &p, const double *C, double *T, unsigned 
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
         return (int) std::min<long long>(items, (long long) num_sms() * std::max(per, 1));
     };
-    if (p.naux % 2 == 0 && p.Cpad) {
+    if (p.naux % 2 == 0 && p.Cpad && wait_word()) {
         const int cp = stiles * K::S, zeros = std::max(K::S, K::P);
         const int n = p.nbf * cp + zeros;
         k_pad_cocc<<<(n + 255) / 256, 256, 0, s>>>(C, p.Cpad, p.nbf, p.nocc, cp, zeros);
@@ -524,7 +516,7 @@ static void launch_half(const FockPlan &p, const double *C, double *T, unsigned 
         const int g = grid(k_halftransform_bulk<WS, NX, WP, NY>, KB::THREADS, KB::SMEM);
         k_halftransform_bulk<WS, NX, WP, NY><<<g, KB::THREADS, KB::SMEM, s>>>(
             p.B, p.Cpad, cp, p.Cpad + (size_t) p.nbf * cp, p.csr_j, p.csr_u, p.csr_displs, p.nocc, p.naux, T,
-            (int) items, stiles, ptiles, rowmax);
+            (int) items, stiles, ptiles, rowmax, wait_word());
     } else {
         const int g = grid(k_halftransform_pipe<WS, NX, WP, NY>, K::THREADS, K::SMEM);
         k_halftransform_pipe<WS, NX, WP, NY><<<g, K::THREADS, K::SMEM, s>>>(p.B, C, p.csr_j, p.csr_u, p.csr_displs, p.nocc,

@@ -40,15 +40,17 @@ constexpr int BK = 64;           // K per pipeline stage (one 128-byte swizzle r
 constexpr int UK = 16;           // K per tcgen05.mma.kind::f16
 constexpr long long WAIT_CYCLES = 4000000000LL;   // ~2 s at 2 GHz
 
-__device__ int g_umma_error;     // set to a nonzero code when a bounded wait times out
+__device__ int *g_umma_flag;     // the process's wait word: gets a nonzero code when a bounded wait times out
 
 using namespace umma;
 
 // Bounded wait on an mbarrier phase (at most `limit` clock cycles). Returns
-// false (and records code in g_umma_error) on timeout.
+// false (and records code in the wait word) on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase, int code, long long limit = WAIT_CYCLES)
 {
-    return mbar_wait_bounded(bar, phase, &g_umma_error, code, limit);
+    if (mbar_try_bounded(bar, phase, limit)) return true;
+    *(volatile int *) g_umma_flag = code;
+    return false;
 }
 
 // kind::f16 instruction descriptor: BF16 x BF16 -> FP32, both K-major, M = 128, N = n.
@@ -1019,6 +1021,9 @@ int kmix_create(KMix **out, const FockPlan &p, const int *h_displs, cudaStream_t
 {
     *out = nullptr;
     if (p.nocc > 256) return ERR_UNSUPPORTED;
+    int *const word = wait_word();
+    if (!word) return ERR_ALLOC;
+    TSCF_CUDA_CHECK(cudaMemcpyToSymbol(g_umma_flag, &word, sizeof(word)));
     KMix *k = new KMix();
     k->nbf = p.nbf;
     k->naux = p.naux;
@@ -1432,13 +1437,6 @@ int kmix_batch_build(KMixBatch *b, const int *active, const double *const *Cocc,
     return cuda_launch_rc("batched tensor-core exchange");
 }
 
-int kmix_error_flag()
-{
-    int v = 0;
-    cudaMemcpyFromSymbol(&v, g_umma_error, sizeof(int));
-    return v;
-}
-
 // The bounded-wait path of the G GEMM kernel, run on purpose: one CTA with
 // no copies issued, so its MMA warp waits on a stage that nothing fills and
 // its epilogue on an accumulator that nothing completes. Both waits give up
@@ -1448,8 +1446,6 @@ int kmix_error_flag()
 int kmix_wait_probe(KMix *k, long long wait_cycles, int *code, cudaStream_t s)
 {
     if (!k || !code || wait_cycles < 0) return ERR_INPUT;
-    const int zero = 0;
-    TSCF_CUDA_CHECK(cudaMemcpyToSymbolAsync(g_umma_error, &zero, sizeof(int), 0, cudaMemcpyHostToDevice, s));
     GArgs ga{k->G, k->nbf, k->chunks_per_split, k->total_chunks};
     ga.probe = 1;
     ga.wait_cycles = wait_cycles;
@@ -1461,8 +1457,7 @@ int kmix_wait_probe(KMix *k, long long wait_cycles, int *code, cudaStream_t s)
     g_launches++;
     TSCF_CUDA_CHECK(cudaGetLastError());
     TSCF_CUDA_CHECK(cudaStreamSynchronize(s));
-    TSCF_CUDA_CHECK(cudaMemcpyFromSymbol(code, g_umma_error, sizeof(int)));
-    TSCF_CUDA_CHECK(cudaMemcpyToSymbol(g_umma_error, &zero, sizeof(int)));
+    *code = waits_take();
     return OK;
 }
 

@@ -111,11 +111,10 @@ constexpr size_t BG_SMEM = sizeof(double) * BG_STAGES * BG_STAGE + 1024;
 constexpr long long BG_WAIT = 2000000000LL;   // clock cycles a barrier wait may take (~1 s)
 static_assert(BG_SMEM + 64 <= 227 * 1024 && BG_M <= 256, "bulk GEMM stages exceed shared memory");
 static_assert(BG_ABOX % 128 == 0 && BG_BBOX % 128 == 0, "swizzled boxes start at multiples of 1024 bytes");
-__device__ int g_gemm_error;
 
 __global__ void __launch_bounds__(BG_THREADS, 1)
     k_dgemm_bulk(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, int m, int n, int k,
-                 double alpha, double *__restrict__ C, int ldc, int ntn, int ntiles)
+                 double alpha, double *__restrict__ C, int ldc, int ntn, int ntiles, int *gave_up)
 {
     extern __shared__ __align__(1024) unsigned char bg_raw[];
     double *bgsm = (double *) (((uintptr_t) bg_raw + 1023) & ~(uintptr_t) 1023);
@@ -137,9 +136,9 @@ __global__ void __launch_bounds__(BG_THREADS, 1)
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
             const int m0 = t / ntn * BG_M, n0 = t % ntn * BG_N;
             for (int k0 = 0; k0 < k; k0 += BG_K) {
-                if (!first && !umma::mbar_wait_bounded(&empty[st], phase ^ 1, &g_gemm_error, 41, BG_WAIT)) {
+                if (!first && !umma::mbar_wait_bounded(&empty[st], phase ^ 1, gave_up, 41, BG_WAIT)) {
                     for (int q = 0; q < BG_STAGES; q++) {   // its copies in flight, oldest first
-                        umma::mbar_wait_bounded(&full[st], phase ^ 1, &g_gemm_error, 42, BG_WAIT);
+                        umma::mbar_wait_bounded(&full[st], phase ^ 1, gave_up, 42, BG_WAIT);
                         if (++st == BG_STAGES) {
                             st = 0;
                             phase ^= 1;
@@ -180,7 +179,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1)
 #pragma unroll
             for (int y = 0; y < BG_NY; y++) acc[x][y][0] = acc[x][y][1] = 0.0;
         for (int k0 = 0; k0 < k; k0 += BG_K) {
-            if (!umma::mbar_wait_bounded(&full[st], phase, &g_gemm_error, 43, BG_WAIT)) return;
+            if (!umma::mbar_wait_bounded(&full[st], phase, gave_up, 43, BG_WAIT)) return;
             const double *As = bgsm + (size_t) st * BG_STAGE, *Bs = As + BG_K / 16 * BG_ABOX;
 #pragma unroll
             for (int k4 = 0; k4 < BG_K; k4 += 4) {   // zeros behind k, m and n
@@ -239,7 +238,7 @@ static bool dgemm_bulk(int m, int n, int k, double alpha, const double *A, int l
                        int ldc, cudaStream_t s)
 {
     CUtensorMap mA, mB;
-    if (!umma::make_map_2d(&mA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, m, k, lda, 16, BG_M) ||
+    if (!wait_word() || !umma::make_map_2d(&mA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, m, k, lda, 16, BG_M) ||
         !umma::make_map_2d(&mB, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, B, k, n, ldb, 16, BG_K))
         return false;
     if (cudaFuncSetAttribute(k_dgemm_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) BG_SMEM) != cudaSuccess) {
@@ -247,16 +246,10 @@ static bool dgemm_bulk(int m, int n, int k, double alpha, const double *A, int l
         return false;
     }
     const int ntn = (n + BG_N - 1) / BG_N, ntiles = ntn * ((m + BG_M - 1) / BG_M);
-    k_dgemm_bulk<<<std::min(ntiles, num_sms()), BG_THREADS, BG_SMEM, s>>>(mA, mB, m, n, k, alpha, C, ldc, ntn, ntiles);
+    k_dgemm_bulk<<<std::min(ntiles, num_sms()), BG_THREADS, BG_SMEM, s>>>(mA, mB, m, n, k, alpha, C, ldc, ntn, ntiles,
+                                                                               wait_word());
     g_launches++;
     return true;
-}
-
-int gemm_error_flag()
-{
-    int v = 0;
-    cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(int));
-    return v;
 }
 
 template <bool TA, bool TB>
@@ -678,6 +671,74 @@ int cuda_launch_rc(const char *what)
     if (err == cudaSuccess) return OK;
     fprintf(stderr, "[tinyscf] CUDA error in %s: %s\n", what, cudaGetErrorString(err));
     return ERR_CUDA;
+}
+
+// ---------------------------------------------------------------- bounded waits
+int *wait_word()
+{
+    static int *const word = [] {
+        int *p = nullptr;
+        if (cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return (int *) nullptr;
+        }
+        *p = 0;
+        return p;
+    }();
+    return word;
+}
+
+static std::mutex g_wait_mu;
+static unsigned g_wait_reports = 0;   // times the word was found set
+static int g_wait_code = 0;           // and what it held the last time
+
+static int take_locked()
+{
+    volatile int *w = wait_word();
+    const int code = w ? *w : 0;
+    if (code) {
+        *w = 0;
+        g_wait_code = code;
+        g_wait_reports++;
+    }
+    return code;
+}
+
+int waits_take()
+{
+    std::lock_guard<std::mutex> lk(g_wait_mu);
+    return take_locked();
+}
+
+unsigned waits_mark()
+{
+    std::lock_guard<std::mutex> lk(g_wait_mu);
+    return g_wait_reports;
+}
+
+int waits_check(unsigned &mark, const char *what)
+{
+    std::lock_guard<std::mutex> lk(g_wait_mu);
+    take_locked();
+    if (g_wait_reports == mark) return OK;
+    mark = g_wait_reports;
+    fprintf(stderr, "[tinyscf] %s: a bounded wait timed out (code %d)\n", what, g_wait_code);
+    return ERR_CUDA;
+}
+
+__global__ void k_wait_probe(long long cycles, int *gave_up)
+{
+    __shared__ uint64_t bar;
+    umma::mbar_init(&bar, 1);
+    umma::mbar_wait_bounded(&bar, 0, gave_up, 71, cycles);
+}
+
+int wait_probe(long long cycles, cudaStream_t s)
+{
+    if (cycles < 0 || !wait_word()) return ERR_INPUT;
+    k_wait_probe<<<1, 1, 0, s>>>(cycles, wait_word());
+    g_launches++;
+    return cudaStreamSynchronize(s) == cudaSuccess ? OK : ERR_CUDA;
 }
 
 // ---------------------------------------------------------------- device memory

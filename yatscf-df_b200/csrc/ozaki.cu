@@ -59,7 +59,6 @@ static_assert(OZ_SMEM <= 227 * 1024, "Ozaki GEMM stages exceed shared memory");
 constexpr long long OZ_WAIT_CYCLES = 4000000000LL;   // ~2 s at 2 GHz
 constexpr double MAGIC = 6755399441055744.0;        // 1.5 * 2^52: x + MAGIC rounds x to an integer
 
-__device__ int g_oz_error;
 __constant__ double c_m[OZ_NMAX], c_inv[OZ_NMAX];
 __constant__ int c_mi[OZ_NMAX], c_y[OZ_NMAX];
 __constant__ unsigned long long c_Mk[OZ_NMAX][2], c_M[2];
@@ -169,6 +168,7 @@ struct OzArgs {
     uint8_t *res;            // [ksplit][nmod][rows_pad][rows_pad] residues of the range sums
     int rows_pad, nmod, chunks_per_split, total_chunks;
     long long wait_cycles;
+    int *gave_up;            // the process's wait word
 };
 
 // One 256 x 256 tile per CTA pair (clusters of 2 along x): CTA r loads rows
@@ -222,7 +222,7 @@ k_oz_gemm(const __grid_constant__ CUtensorMap mR, OzArgs a)
         bool ok = true;
         for (int it = 0; it < nit && ok; it++) {
             const int s = it % OZ_STAGES, k = it / nk, kb = it % nk;
-            if (it >= OZ_STAGES) ok = mbar_wait_bounded(&empty[s], ((it / OZ_STAGES) - 1) & 1, &g_oz_error, 21,
+            if (it >= OZ_STAGES) ok = mbar_wait_bounded(&empty[s], ((it / OZ_STAGES) - 1) & 1, a.gave_up, 21,
                                                         a.wait_cycles);
             if (!ok) break;
             if (rank == 0) mbar_expect_tx(&full[s], 2 * OZ_STAGE_BYTES);
@@ -234,19 +234,19 @@ k_oz_gemm(const __grid_constant__ CUtensorMap mR, OzArgs a)
         }
         // the pair's MMAs have consumed (so the copies have landed in) the last stages
         for (int it = (nit > OZ_STAGES ? nit - OZ_STAGES : 0); it < nit && ok; it++)
-            mbar_wait_bounded(&empty[it % OZ_STAGES], (it / OZ_STAGES) & 1, &g_oz_error, 22, a.wait_cycles);
+            mbar_wait_bounded(&empty[it % OZ_STAGES], (it / OZ_STAGES) & 1, a.gave_up, 22, a.wait_cycles);
     } else if (warp == 1 && lane == 0 && rank == 0) {
         bool ok = true;
         int it = 0;
         for (int k = 0; k < a.nmod && ok && nk > 0; k++) {
             const int b = k & 1;
-            if (k >= 2) ok = mbar_wait_bounded(&tempty[b], ((k >> 1) - 1) & 1, &g_oz_error, 23, a.wait_cycles);
+            if (k >= 2) ok = mbar_wait_bounded(&tempty[b], ((k >> 1) - 1) & 1, a.gave_up, 23, a.wait_cycles);
             if (!ok) break;
             fence_after_sync();
             const uint32_t acc = tmem + b * ON;
             for (int kb = 0; kb < nk && ok; kb++, it++) {
                 const int s = it % OZ_STAGES;
-                ok = mbar_wait_bounded(&full[s], (it / OZ_STAGES) & 1, &g_oz_error, 24, a.wait_cycles);
+                ok = mbar_wait_bounded(&full[s], (it / OZ_STAGES) & 1, a.gave_up, 24, a.wait_cycles);
                 if (!ok) break;
                 fence_after_sync();
                 const uint32_t sa = smem_u32(smem + s * OZ_STAGE_BYTES), sb = sa + OZ_A_BYTES;
@@ -266,7 +266,7 @@ k_oz_gemm(const __grid_constant__ CUtensorMap mR, OzArgs a)
         bool ok = true;
         for (int k = 0; k < a.nmod && ok && nk > 0; k++) {
             const int b = k & 1;
-            ok = mbar_wait_bounded(&tfull[b], (k >> 1) & 1, &g_oz_error, 25, a.wait_cycles);
+            ok = mbar_wait_bounded(&tfull[b], (k >> 1) & 1, a.gave_up, 25, a.wait_cycles);
             if (!ok) break;
             fence_after_sync();
             const int m = c_mi[k];
@@ -462,6 +462,7 @@ int oz_create(OzSyrk **out, int nbf, long long Q, cudaStream_t s)
 {
     *out = nullptr;
     if (nbf <= 0 || Q <= 0) return ERR_INPUT;
+    if (!wait_word()) return ERR_ALLOC;
     OzSyrk *o = new OzSyrk();
     o->nbf = nbf;
     o->Q = Q;
@@ -529,7 +530,7 @@ int oz_syrk(OzSyrk *o, const double *d_T, double *d_K, cudaStream_t s, const uns
     if (d_rowmax) k_oz_exp_from_max<<<(o->nbf + 255) / 256, 256, 0, s>>>(d_rowmax, o->nbf, o->e);
     else k_oz_rowexp<<<o->nbf, 1024, 0, s>>>(d_T, o->Q, o->e);
     k_oz_residues<<<o->nsm * 8, 256, 0, s>>>(d_T, o->nbf, o->Q, o->Qp, o->rows_pad, o->e, o->beta, o->nmod, o->R);
-    OzArgs a{o->tiles, o->res, o->rows_pad, o->nmod, o->cps, o->total_chunks, OZ_WAIT_CYCLES};
+    OzArgs a{o->tiles, o->res, o->rows_pad, o->nmod, o->cps, o->total_chunks, OZ_WAIT_CYCLES, wait_word()};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * o->ntiles, o->ksplit);
     cfg.blockDim = dim3(OZ_THREADS);
@@ -551,12 +552,6 @@ int oz_syrk(OzSyrk *o, const double *d_T, double *d_K, cudaStream_t s, const uns
     return cuda_launch_rc("Ozaki rank-k product");
 }
 
-int oz_error_flag()
-{
-    int v = 0;
-    cudaMemcpyFromSymbol(&v, g_oz_error, sizeof(int));
-    return v;
-}
 
 void oz_info(const OzSyrk *o, int info[6])
 {

@@ -313,6 +313,7 @@ struct Engine {
     bool d_from_cocc = false;   // D = Cocc Cocc^T (set by the engine's density builds, cleared by SAD / set_density)
     OzSyrk *oz = nullptr;   // K = T T^T on the integer tensor cores (used when kozaki)
     bool kozaki = false;
+    unsigned wait_mark = waits_mark();   // of the public call under way (enter)
     long long n_ozaki = 0;  // K = T T^T builds that ran on the integer tensor cores
     double *Jt = nullptr, *Jpart = nullptr, *Jw = nullptr;
     int jblk = 1, jblk_max = 1;
@@ -466,7 +467,7 @@ int sync_rc(Engine *e, const char *what)
         fprintf(stderr, "[tinyscf] CUDA error in %s: %s\n", what, cudaGetErrorString(err));
         return ERR_CUDA;
     }
-    return OK;
+    return waits_check(e->wait_mark, what);   // a kernel that gave up waiting left its output incomplete
 }
 
 int upload_shells(Engine *e, const HostShells &h, int maxl, DevArrays &d)
@@ -1261,10 +1262,6 @@ int df_impl(TinySCF_t t)
     tstop(e, TINYSCF_T_DFGEMM);
     RC(cuda_rc("DF tensor GEMM"));
     int rc = sync_rc(e, "DF tensor");
-    if (const int fl = rc ? 0 : gemm_error_flag()) {
-        fprintf(stderr, "[tinyscf] DF tensor GEMM: a bounded wait timed out (code %d)\n", fl);
-        rc = ERR_CUDA;
-    }
     eig_destroy(eg);
     dfree(e, pqA);
     dfree(e, Jpq);
@@ -1586,12 +1583,14 @@ int graph_iteration(TinySCF_t t, double *E)
 constexpr int kGuardRises = 4;
 constexpr double kGuardRise = 1e-6;
 
+int reset_impl(TinySCF_t t);
+
 int restart_from_sad(TinySCF_t t)
 {
     Engine *e = E_(t);
     const int mode = e->guess_mode;
     e->guess_mode = TINYSCF_GUESS_SAD;
-    const int rc = TinySCF_reset_scf(t);
+    const int rc = reset_impl(t);
     e->guess_mode = mode;
     e->guard_restarts++;
     return rc;
@@ -1683,26 +1682,6 @@ int scf_impl(TinySCF_t t)
             printf("* Final FP64 Fock build: Energy = %.10lf (%.10lf), mixed-precision energy was %.10lf\n",
                    E + t->nuc_energy, E, t->HF_energy + t->nuc_energy);
         t->HF_energy = E;
-        int fl = kmix_error_flag();
-        if (fl) {
-            fprintf(stderr, "[tinyscf] tensor-core K: a bounded wait timed out (code %d)\n", fl);
-            return ERR_CUDA;
-        }
-    }
-    if (const int fl = half_error_flag()) {
-        fprintf(stderr, "[tinyscf] exchange half-transform: a bounded wait timed out (code %d)\n", fl);
-        return ERR_CUDA;
-    }
-    if (const int fl = gemm_error_flag()) {
-        fprintf(stderr, "[tinyscf] FP64 GEMM: a bounded wait timed out (code %d)\n", fl);
-        return ERR_CUDA;
-    }
-    if (e->oz) {
-        const int fl = oz_error_flag();
-        if (fl) {
-            fprintf(stderr, "[tinyscf] integer tensor-core K: a bounded wait timed out (code %d)\n", fl);
-            return ERR_CUDA;
-        }
     }
     cudaEventRecord(scf1, e->s);
     cudaEventSynchronize(scf1);
@@ -1809,10 +1788,17 @@ const char *TinySCF_status_string(int status)
     }
 }
 
+// A public call starts: waits that earlier calls reported are not its own.
+static void enter(TinySCF_t t)
+{
+    if (t->dev) E_(t)->wait_mark = waits_mark();
+}
+
 #define STATUS_WRAP(name, call)            \
     int name(TinySCF_t t)                  \
     {                                      \
         if (!t) return TINYSCF_ERR_STATE;  \
+        enter(t);                          \
         int rc = (call);                   \
         t->status = rc;                    \
         return rc;                         \
@@ -1868,6 +1854,7 @@ int TinySCF_set_fock(TinySCF_t t, const double *F, int orthogonal)
 int TinySCF_sync_host(TinySCF_t t)
 {
     if (!t || !t->dev) return TINYSCF_ERR_STATE;
+    enter(t);
     return sync_host_impl(t);
 }
 
@@ -1892,6 +1879,7 @@ int TinySCF_set_k_precision(TinySCF_t t, int mode)
     if (!t || !t->dev) return TINYSCF_ERR_STATE;
     Engine *e = E_(t);
     if (mode != TINYSCF_K_FP64 && mode != TINYSCF_K_MIXED) return TINYSCF_ERR_INPUT;
+    enter(t);
     if (mode == TINYSCF_K_MIXED) {
         if (e->stage < 5) return TINYSCF_ERR_STATE;   // needs the DF tensor
         if (!e->kmix) {
@@ -2074,6 +2062,16 @@ int TinySCF_guess_mlp_grad(int din, int hid, int dout, const float *params, cons
 int TinySCF_reset_scf(TinySCF_t t)
 {
     if (!t || !t->dev) return TINYSCF_ERR_STATE;
+    enter(t);
+    return reset_impl(t);
+}
+
+}  // extern "C"
+
+namespace {
+
+int reset_impl(TinySCF_t t)
+{
     Engine *e = E_(t);
     if (e->stage < 4) return TINYSCF_ERR_STATE;
     int verbose = t->verbose;
@@ -2092,6 +2090,10 @@ int TinySCF_reset_scf(TinySCF_t t)
     t->DIIS_bmax = -DBL_MAX;
     return sync_rc(e, "reset");
 }
+
+}  // namespace
+
+extern "C" {
 
 int TinySCF_get_timing_stats(TinySCF_t t, double *sum_ms, long long *count, int n)
 {
@@ -2477,6 +2479,8 @@ int batch_refine(TinySCF_batch_t b, const std::vector<int> &todo, std::vector<in
 int batch_scf_impl(TinySCF_batch_t b)
 {
     const int nmol = (int) b->mols.size();
+    unsigned mark = waits_mark();
+    for (TinySCF_t t : b->mols) E_(t)->wait_mark = mark;
     std::vector<int> act(nmol, 0);
     std::vector<double> prev(nmol, 0.0), delta(nmol, 223.0), Eh(nmol, 0.0);
     for (int k = 0; k < nmol; k++) {
@@ -2574,6 +2578,7 @@ int batch_scf_impl(TinySCF_batch_t b)
             b->phase_ms[q] += pm;
         }
         TSCF_CUDA_CHECK(cudaGetLastError());
+        RC(waits_check(mark, "batched SCF iteration"));
         for (int k = 0; k < nmol; k++) {
             if (!act[k]) continue;
             TinySCF_t t = b->mols[k];
@@ -2609,11 +2614,7 @@ int batch_scf_impl(TinySCF_batch_t b)
         b->phase_ms[5] += pm;
         for (int k = 0; k < nmol; k++)
             if (b->mixed[k]) b->mols[k]->HF_energy = Eh[k];
-        const int fl = kmix_error_flag();
-        if (fl) {
-            fprintf(stderr, "[tinyscf] tensor-core K: a bounded wait timed out (code %d)\n", fl);
-            return ERR_CUDA;
-        }
+        RC(waits_check(mark, "batched SCF, final FP64 Fock builds"));
     }
     cudaEventRecord(b->ev1, b->s);
     TSCF_CUDA_CHECK(cudaEventSynchronize(b->ev1));
@@ -2756,6 +2757,7 @@ int TinySCF_set_JK(TinySCF_t t, const double *J, const double *K)
     if (!t || !t->dev || !J || !K) return TINYSCF_ERR_STATE;
     Engine *e = E_(t);
     if (e->stage < 5) return TINYSCF_ERR_STATE;
+    enter(t);
     const size_t bytes = sizeof(double) * e->nn;
     if (cudaMemcpyAsync(e->J, J, bytes, cudaMemcpyHostToDevice, e->s) != cudaSuccess ||
         cudaMemcpyAsync(e->K, K, bytes, cudaMemcpyHostToDevice, e->s) != cudaSuccess)
@@ -2783,6 +2785,12 @@ int TinySCF_kmix_wait_probe(TinySCF_t t, long long wait_cycles, int *code)
     return kmix_wait_probe(e->kmix, wait_cycles, code, e->s);
 }
 
+int TinySCF_wait_probe(TinySCF_t t, long long wait_cycles)
+{
+    if (!t || !t->dev) return TINYSCF_ERR_STATE;
+    return wait_probe(wait_cycles, E_(t)->s);
+}
+
 int TinySCF_eigh(int device, int n, const double *A, double *w, double *V)
 {
     if (n < 1 || n > EIG_MAX_N || !A || !w || !V) return TINYSCF_ERR_INPUT;
@@ -2799,12 +2807,13 @@ int TinySCF_eigh(int device, int n, const double *A, double *w, double *V)
     } else if (cudaMemcpyAsync(dA, A, sizeof(double) * nn, cudaMemcpyHostToDevice, s) != cudaSuccess) {
         rc = TINYSCF_ERR_CUDA;
     } else {
+        unsigned mark = waits_mark();
         rc = eig_run(eg, dA, dw, dV, s, true);
         if (rc == OK && (cudaMemcpyAsync(w, dw, sizeof(double) * n, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaMemcpyAsync(V, dV, sizeof(double) * nn, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaStreamSynchronize(s) != cudaSuccess))
             rc = TINYSCF_ERR_CUDA;
-        if (rc == OK) rc = eig_error(eg);
+        if (rc == OK) rc = waits_check(mark, "eigensolver");
     }
     eig_destroy(eg);
     cudaFree(dA);
@@ -2835,6 +2844,7 @@ int TinySCF_syrk_int8(int device, int n, long long q, const double *T, double *K
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return TINYSCF_ERR_CUDA;
     double *dT = nullptr, *dK = nullptr;
     OzSyrk *oz = nullptr;
+    unsigned mark = waits_mark();
     int rc = TINYSCF_OK;
     if (cudaMalloc(&dT, sizeof(double) * (size_t) n * q) != cudaSuccess ||
         cudaMalloc(&dK, sizeof(double) * (size_t) n * n) != cudaSuccess) {
@@ -2847,7 +2857,7 @@ int TinySCF_syrk_int8(int device, int n, long long q, const double *T, double *K
                  (cudaMemcpyAsync(K, dK, sizeof(double) * (size_t) n * n, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                   cudaStreamSynchronize(s) != cudaSuccess))
             rc = TINYSCF_ERR_CUDA;
-        if (rc == OK && oz_error_flag()) rc = TINYSCF_ERR_CUDA;
+        if (rc == OK) rc = waits_check(mark, "integer rank-k product");
     }
     oz_destroy(oz);
     cudaFree(dT);

@@ -120,7 +120,19 @@ int device_bf_fill(const double *d_bf_scr, int n, double eta, const int *d_work,
 void dgemm(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda,
            const double *B, int ldb, double beta, double *C, int ldc, cudaStream_t s);
 
-int gemm_error_flag();   // nonzero: a bounded wait of k_dgemm_bulk gave up
+// Bounded waits. A kernel whose wait gives up stores a code to one page-locked
+// word of the process and returns with its output incomplete. Whoever waits for
+// a stream asks waits_check: an error if the word is set, or was found set by
+// another call, since the call took its mark from waits_mark (two calls at once
+// cannot tell whose kernel it was: both fail). The word is cleared as it is
+// reported, so the next call starts clean. No copy and no launch: the host reads
+// its own memory.
+int     *wait_word();   // the word's address for the kernels (every device); nullptr: none to be had
+unsigned waits_mark();
+int      waits_check(unsigned &mark, const char *what);
+int      waits_take();   // the word's code (0: none), taken as reported
+// Stores the code of a wait that runs out after `cycles` (a barrier that nothing completes), to test the reports.
+int      wait_probe(long long cycles, cudaStream_t s);
 // The same product with the tile picked from the call shape (no tuning run).
 void dgemm_untuned(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda,
                    const double *B, int ldb, double beta, double *C, int ldc, cudaStream_t s);
@@ -145,16 +157,15 @@ int  dev_trim(int device);   // return the pool's unused memory to the device
 // Symmetric eigen-decomposition (eigh.cu; ascending eigenvalues). A is
 // row-major n x n symmetric; on return V holds eigenvectors as ROWS (V[k*n + i]
 // = i-th entry of eigenvector k); V may alias A. Workspace (four n x n
-// matrices) is owned by the Eig object; n <= EIG_MAX_N. Asynchronous on s;
-// eig_error() (synchronous) reports a grid barrier of the tridiagonalisation
-// that gave up waiting.
+// matrices) is owned by the Eig object; n <= EIG_MAX_N. Asynchronous on s; a
+// grid barrier of the tridiagonalisation that gave up waiting shows in
+// waits_check().
 constexpr int EIG_MAX_N = 8192;
 struct Eig;
 Eig *eig_create(int n, cudaStream_t s);
 void eig_destroy(Eig *e);
 // at_noise: the secular equation's roots stop where its value is rounding (k_dc_secular).
 int  eig_run(Eig *e, const double *d_A, double *d_w, double *d_V, cudaStream_t s, bool at_noise = false);
-int  eig_error(Eig *e);
 // Whether every panel runs as one cluster (no cooperative launch that needs all the chip).
 bool eig_small_launches(const Eig *e);
 
@@ -215,7 +226,6 @@ void convert_f32(const double *in, float *out, size_t n, cudaStream_t s);
 void build_K_halftransform(const FockPlan &p, const double *d_Cocc, double *d_T, cudaStream_t s, int wide = 0,
                            unsigned long long *d_rowmax = nullptr);
 size_t half_pad_elems(int nbf, int nocc);
-int    half_error_flag();   // nonzero: a bounded wait of the half-transform gave up
 // ... then K = T T^T over upper 64x64 tiles (d_tiles: (bi,bj), bi <= bj), split-K, mirrored.
 // tile = 64 (k_syrk_part, FFMA), 128 (k_syrk_part128, FFMA) or KSYRK_DMMA
 // (k_syrk_dmma: 128 x 128 tiles on the FP64 tensor cores); d_tiles lists the
@@ -239,7 +249,6 @@ void kmix_reset(KMix *k, cudaStream_t s);
 // it and the G GEMM, 2 after the G GEMM (device timers around the two).
 int  kmix_build(KMix *k, const double *Cocc, const double *S, double *K, cudaStream_t s,
                 const std::function<void(int)> &mark = nullptr);
-int  kmix_error_flag();
 // Many molecules' incremental K builds with one half-transform launch and one
 // G GEMM launch over all of them (the alignments and reductions stay per
 // molecule). ks: the molecules' KMix objects (owned by the caller).
@@ -263,7 +272,6 @@ void oz_destroy(OzSyrk *o);
 // else nullptr (the rows are scanned).
 int  oz_syrk(OzSyrk *o, const double *d_T, double *d_K, cudaStream_t s, const unsigned long long *d_rowmax = nullptr);
 unsigned long long *oz_rowmax(OzSyrk *o);
-int  oz_error_flag();
 // {moduli, beta, tiles, K ranges, chunks per range, padded rows}
 void oz_info(const OzSyrk *o, int info[6]);
 

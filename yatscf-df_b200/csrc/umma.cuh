@@ -29,9 +29,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Bounded wait on an mbarrier phase (at most `limit` clock cycles). On timeout
-// writes `code` to *flag and returns false.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t phase, int *flag, int code, long long limit)
+// Bounded wait on an mbarrier phase (at most `limit` clock cycles): whether it completed.
+__device__ __forceinline__ bool mbar_try_bounded(uint64_t *bar, uint32_t phase, long long limit)
 {
     const uint32_t addr = smem_u32(bar);
     const long long t0 = clock64();
@@ -45,11 +44,16 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t phase,
             : "r"(addr), "r"(phase)
             : "memory");
         if (done) return true;
-        if (clock64() - t0 > limit) {
-            atomicExch(flag, code);
-            return false;
-        }
+        if (clock64() - t0 > limit) return false;
     }
+}
+
+// The same; a wait that gives up writes `code` to *flag (the process's wait word, wait_word()).
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t phase, int *flag, int code, long long limit)
+{
+    if (mbar_try_bounded(bar, phase, limit)) return true;
+    *(volatile int *) flag = code;
+    return false;
 }
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y)

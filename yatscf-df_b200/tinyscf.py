@@ -131,6 +131,7 @@ def load_library(path=LIBPATH):
         "TinySCF_syrk_int8": ([ip, ip, ctypes.c_longlong, dp, dp], ip),
         "TinySCF_trim_memory": ([ip], ip),
         "TinySCF_kmix_wait_probe": ([T, ctypes.c_longlong, ctypes.POINTER(ctypes.c_int)], ip),
+        "TinySCF_wait_probe": ([T, ctypes.c_longlong], ip),
         "TinySCF_set_aux_slice": ([T, ip, ip], ip),
         "TinySCF_set_JK": ([T, dp, dp], ip),
     }
@@ -348,6 +349,12 @@ class TinySCF:
         if rc:
             raise TinySCFError("kmix_wait_probe: " + STATUS.get(rc, str(rc)))
         return code.value
+
+    def wait_probe(self, wait_cycles):
+        """Run one bounded wait out (wait_cycles clock cycles) and leave it for the next call to report."""
+        rc = self.lib.TinySCF_wait_probe(self.t, int(wait_cycles))
+        if rc:
+            raise TinySCFError("wait_probe: " + STATUS.get(rc, str(rc)))
 
     def reset_scf(self):
         rc = self.lib.TinySCF_reset_scf(self.t)
