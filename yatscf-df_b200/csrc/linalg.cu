@@ -602,6 +602,28 @@ int ns_inv_sqrt(const double *d_M, double *d_Z, int o, int iters, cudaStream_t s
     return OK;
 }
 
+// Whether a tuned product goes to the K-split tile. Every other tile sums over k
+// in one chain, so they may be timed against one another; the K-split tile rounds
+// differently, and the accelerated solve turns 1e-16 in X, or in a refinement
+// product, into 1e-9 of its density. Timed against the others it won or lost by a
+// coin toss near the line (1010^3 with A transposed: 0.147 ms both; 585 x 93 x 93:
+// 9.7 us both), so C40H82's density differed by 2-5e-9 from process to process.
+// The line lies where its advantage ends, at 6 (A transposed), 4 (B transposed)
+// or 5 of its CTAs an SM; times of the K-split tile over the best other one: A
+// transposed 760^3 0.67, 910^3 0.92 (841 CTAs), 935^3 1.01 (900), 1152^3 1.09;
+// plain 760^3 0.93, 835^3 0.98 (729), 885^3 1.09 (784); B transposed
+// 760 x 760 x 121 0.88 (576), 835 x 835 x 133 1.08 (729), with a long K
+// 835 x 835 x 266 0.96 (729), 885 x 885 x 282 1.02 (784). At the other end few CTAs
+// with one K chunk and a half have nothing to split: 400 x 80 x 80 1.26,
+// 510 x 81 x 81 1.12, 500 x 100 x 100 0.90.
+static bool ksplit_order(bool ta, bool tb, int m, int n, int k)
+{
+    const long long tiles = (long long) ((m + KS_T - 1) / KS_T) * ((n + KS_T - 1) / KS_T);
+    if (k < 100 && tiles < 64) return false;
+    const int per = ta ? 6 : (!tb || k >= 256) ? 5 : 4;
+    return tiles <= (long long) per * num_sms();
+}
+
 void dgemm(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda, const double *B, int ldb,
            double beta, double *C, int ldc, cudaStream_t s)
 {
@@ -623,7 +645,12 @@ void dgemm(bool ta, bool tb, int m, int n, int k, double alpha, const double *A,
         const size_t ea = ta ? (size_t) k * lda : (size_t) m * lda, eb = tb ? (size_t) n * ldb : (size_t) k * ldb;
         if (tune_enabled() && cs == cudaStreamCaptureStatusNone && beta == 0.0 && disjoint(A, ea) && disjoint(B, eb) &&
             (double) m * n * k >= 2e6) {
-            v = tune_run(key, {0, 1, 2, 3, 4, 5}, [&](int c) { dgemm_variant(c, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s); }, s);
+            if (ksplit_order(ta, tb, m, n, k)) {
+                tune_fix(key, 5);
+                dgemm_variant(5, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s);
+                return;
+            }
+            v = tune_run(key, {0, 1, 2, 3, 4}, [&](int c) { dgemm_variant(c, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s); }, s);
             return;
         }
         if (beta == 0.0 && (double) m * n * k < 2e6) {

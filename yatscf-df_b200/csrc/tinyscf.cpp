@@ -1197,12 +1197,13 @@ int autotune_fock(TinySCF_t t)
     snprintf(key, sizeof(key), "jrows:%d:%d", e->nup, t->df_nbf);
     c = tune_lookup(key);
     if (c < 0) {
-        std::vector<int> cand;
+        // by a rule, not by timing: the count is the order of J's sums (see ksplit_order). One block an SM up
+        // to 5.2e6 elements of B (us on 148 / 296 / 592 blocks: 4.5e6 38 / 42 / 57, 6.0e6 43.5 / 42.5 / 58), two
+        // beyond (1.1e7 83 / 67 / 75, 4.8e8 2114 / 1530 / 1581)
         const int nsm = num_sms();
-        for (int v : {nsm, 2 * nsm, 4 * nsm})
-            if (v <= e->jblk_max && std::find(cand.begin(), cand.end(), v) == cand.end()) cand.push_back(v);
-        if (cand.empty()) cand.push_back(e->jblk);
-        c = tune_run(key, cand, [&](int nb) { build_J(p, e->D, e->J, e->Jt, e->Jpart, nb, e->Jw, e->s); }, e->s);
+        c = (double) e->nup * t->df_nbf <= 5.2e6 ? nsm : 2 * nsm;
+        if (c > e->jblk_max) c = e->jblk;
+        tune_fix(key, c);
     }
     if (c >= 1 && c <= e->jblk_max) e->jblk = c;
     return sync_rc(e, "autotuning");

@@ -107,6 +107,14 @@ int tune_run(const std::string &key, const std::vector<int> &cands, const std::f
     return best;
 }
 
+void tune_fix(const std::string &key, int choice)
+{
+    std::lock_guard<std::mutex> lk(g_mu);
+    load_file_locked();
+    g_table[key] = Entry{choice, 0.0, {}};
+    save_file_locked();
+}
+
 std::string tune_report()
 {
     std::lock_guard<std::mutex> lk(g_mu);
