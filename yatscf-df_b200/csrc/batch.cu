@@ -294,7 +294,8 @@ void diis_solve_batched(const MolDev *d_mols, const int *d_active, int nmol, cud
 void batch_j(const BatchPlan &b, cudaStream_t s, int use32)
 {
     const size_t shm = sizeof(double) * b.naux_max;
-    if (shm > 48 * 1024) cudaFuncSetAttribute(kb_j_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
+    if (shm > 48 * 1024)
+        cudaFuncSetAttribute(kb_j_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(double) * MAX_NAUX);
     kb_j_weights<<<b.nup256.total, 256, 0, s>>>(b.mols, b.active, b.nup256);
     kb_j_tpart<<<b.jblk.total, JT_THREADS, 0, s>>>(b.mols, b.active, b.jblk, use32);
     kb_j_treduce<<<b.naux256.total, 256, 0, s>>>(b.mols, b.active, b.naux256);

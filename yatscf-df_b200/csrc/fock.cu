@@ -103,7 +103,8 @@ static void build_J_t(const FockPlan &p, const BT *B, const double *d_D, double 
     k_j_treduce<<<(p.naux + 63) / 64, 64, 0, s>>>(d_part, nblk, p.naux, d_t);
     int blocks = num_sms() * 4;
     const size_t shm = sizeof(double) * p.naux;   // t(P) staged in shared memory
-    if (shm > 48 * 1024) cudaFuncSetAttribute(k_j_rows<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) shm);
+    if (shm > 48 * 1024)   // the largest naux's: a limit is the kernel's, other threads launch it too
+        cudaFuncSetAttribute(k_j_rows<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(double) * MAX_NAUX);
     k_j_rows<BT><<<blocks, 256, shm, s>>>(B, p.up_i, p.up_j, p.up_u, d_t, p.nup, p.naux, p.nbf, d_J);
 }
 

@@ -1231,14 +1231,14 @@ static int launch_gemm(const KMix *k, const GArgs &ga, cudaStream_t s)
 // One incremental K build from the new occupied factor Cocc (nbf x nocc).
 // Alignment of the new occupied factor and the gathered dC operands of one
 // molecule (everything of an incremental K build before the half-transform).
-static void kmix_prepare(KMix *k, const double *Cocc, const double *S, cudaStream_t s)
+static int kmix_prepare(KMix *k, const double *Cocc, const double *S, cudaStream_t s)
 {
     const int n = k->nbf, o = k->nocc;
     // align C_n to C_{n-1}: R = polar(C_n^T S C_{n-1}) by Newton-Schulz; R = I if it does not converge
     dgemm(false, false, n, o, n, 1.0, S, n, k->Cprev, o, 0.0, k->SC, o, s);
     dgemm(true, false, o, o, n, 1.0, Cocc, o, k->SC, o, 0.0, k->X, o, s);
     if (ns_fits(o)) {
-        ns_polar(k->X, k->Y, o, 12, s);
+        if (const int rc = ns_polar(k->X, k->Y, o, 12, s)) return rc;
     } else {
         for (int it = 0; it < 12; it++) {
             dgemm(true, false, o, o, o, 1.0, k->X, o, k->X, o, 0.0, k->Y, o, s);
@@ -1256,6 +1256,7 @@ static void kmix_prepare(KMix *k, const double *Cocc, const double *S, cudaStrea
     k_gather_dc<<<(unsigned) ((k->rp + GD_R - 1) / GD_R), 256, 0, s>>>(k->dC, k->pad_entry, k->csr_j, o, k->rp,
                                                                        k->bn_half, k->Ch, k->Cl);
     g_launches += 3;
+    return OK;
 }
 
 // K += sym(sum over the first nsplit splits of G) (the first build of a solve sets K).
@@ -1278,9 +1279,9 @@ static HalfArgs half_args(const KMix *k)
 int kmix_build(KMix *k, const double *Cocc, const double *S, double *K, cudaStream_t s,
                const std::function<void(int)> &mark)
 {
-    kmix_prepare(k, Cocc, S, s);
+    int rc = kmix_prepare(k, Cocc, S, s);
+    if (rc) return rc;
     HalfArgs ha = half_args(k);
-    int rc;
     if (mark) mark(0);
     switch (k->bn_half) {
     case 16: rc = launch_half<16>(k, ha, s); break;
@@ -1393,7 +1394,8 @@ int kmix_batch_build(KMixBatch *b, const int *active, const double *const *Cocc,
     }
     if (hh[n] == 0) return OK;
     for (int m = 0; m < n; m++)
-        if (active[m]) kmix_prepare(b->ks[m], Cocc[m], S[m], s);
+        if (active[m])
+            if (const int rc = kmix_prepare(b->ks[m], Cocc[m], S[m], s)) return rc;
     TSCF_CUDA_CHECK(cudaMemcpyAsync(b->d_starts, hh, sizeof(int) * 2 * (n + 1), cudaMemcpyHostToDevice, s));
     {
         constexpr int SMEM = kb_half_smem_bytes();

@@ -584,22 +584,29 @@ static size_t ns_smem(int o, int mats)
 
 bool ns_fits(int o) { return o >= 1 && o <= NS_MAX; }
 
+// The limit is a kernel's, not a launch's: every caller sets the largest size's, or a thread with a
+// smaller molecule could lower it under another thread's launch.
+template <class F>
+static int ns_limit(F kernel, int mats)
+{
+    TSCF_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) ns_smem(NS_MAX, mats)));
+    return OK;
+}
+
 int ns_polar(double *d_X, double *d_Y, int o, int iters, cudaStream_t s)
 {
-    const int bytes = (int) ns_smem(o, 3);
-    TSCF_CUDA_CHECK(cudaFuncSetAttribute(k_ns_polar, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    k_ns_polar<<<1, NS_THREADS, bytes, s>>>(d_X, d_Y, o, iters);
+    if (const int rc = ns_limit(k_ns_polar, 3)) return rc;
+    k_ns_polar<<<1, NS_THREADS, ns_smem(o, 3), s>>>(d_X, d_Y, o, iters);
     g_launches++;
-    return OK;
+    return cuda_launch_rc("polar factor");
 }
 
 int ns_inv_sqrt(const double *d_M, double *d_Z, int o, int iters, cudaStream_t s)
 {
-    const int bytes = (int) ns_smem(o, 4);
-    TSCF_CUDA_CHECK(cudaFuncSetAttribute(k_ns_inv_sqrt, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    k_ns_inv_sqrt<<<1, NS_THREADS, bytes, s>>>(d_M, d_Z, o, iters);
+    if (const int rc = ns_limit(k_ns_inv_sqrt, 4)) return rc;
+    k_ns_inv_sqrt<<<1, NS_THREADS, ns_smem(o, 4), s>>>(d_M, d_Z, o, iters);
     g_launches++;
-    return OK;
+    return cuda_launch_rc("inverse square root");
 }
 
 // Whether a tuned product goes to the K-split tile. Every other tile sums over k

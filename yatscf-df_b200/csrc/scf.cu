@@ -428,12 +428,9 @@ __global__ void k_eye(double *A, int n)
 }
 
 // M^-1/2 of an SPD matrix close to I (coupled Newton-Schulz), result in Z.
-static void inv_sqrt_ns(const double *M, double *Y, double *Z, double *T, double *W, int o, int iters, cudaStream_t s)
+static int inv_sqrt_ns(const double *M, double *Y, double *Z, double *T, double *W, int o, int iters, cudaStream_t s)
 {
-    if (ns_fits(o)) {
-        ns_inv_sqrt(M, Z, o, iters, s);
-        return;
-    }
+    if (ns_fits(o)) return ns_inv_sqrt(M, Z, o, iters, s);
     const unsigned nb = (unsigned) ((o * o + 255) / 256);
     cudaMemcpyAsync(Y, M, sizeof(double) * o * o, cudaMemcpyDeviceToDevice, s);
     k_eye<<<nb, 256, 0, s>>>(Z, o);
@@ -447,6 +444,7 @@ static void inv_sqrt_ns(const double *M, double *Y, double *Z, double *T, double
         cudaMemcpyAsync(Z, W, sizeof(double) * o * o, cudaMemcpyDeviceToDevice, s);
         g_launches++;
     }
+    return OK;
 }
 
 // res = max|R|, R = (I - U^T U) F' U^T; UA = U F' U^T
@@ -462,8 +460,8 @@ void subspace_residual(const double *d_Fp, const double *d_U, int n, int o, Subs
 }
 
 // one preconditioned step on U followed by Loewdin re-orthonormalisation
-void subspace_update(const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o, SubspaceWork &w,
-                     cudaStream_t s)
+int subspace_update(const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o, SubspaceWork &w,
+                    cudaStream_t s)
 {
     const int v = n - o;
     const double *Vv = d_Vstale + (size_t) o * n;
@@ -473,10 +471,11 @@ void subspace_update(const double *d_Vstale, const double *d_wstale, double *d_U
     dgemm(true, false, n, o, v, 1.0, Vv, n, w.Cv, o, 0.0, w.A, o, s);         // A = Vv^T Cv (n x o)
     k_add_transposed<<<(unsigned) (((size_t) o * n + 255) / 256), 256, 0, s>>>(d_U, w.A, o, n);
     dgemm(false, true, o, o, n, 1.0, d_U, n, d_U, n, 0.0, w.M, o, s);         // M = U U^T
-    inv_sqrt_ns(w.M, w.Y, w.Z, w.T, w.W, o, 5, s);                              // Z = M^-1/2
+    if (const int rc = inv_sqrt_ns(w.M, w.Y, w.Z, w.T, w.W, o, 5, s)) return rc;   // Z = M^-1/2
     dgemm(false, false, o, n, o, 1.0, w.Z, o, d_U, n, 0.0, w.A, n, s);        // U = Z U
     cudaMemcpyAsync(d_U, w.A, sizeof(double) * (size_t) o * n, cudaMemcpyDeviceToDevice, s);
     g_launches += 2;
+    return OK;
 }
 
 // Stop rule shared by the host loop and the graph's device-side loop: stop when
@@ -505,7 +504,7 @@ int subspace_refine(const double *d_Fp, const double *d_Vstale, const double *d_
         if (cudaStreamSynchronize(s) != cudaSuccess) return ERR_CUDA;
         if (!refine_continue(res, prev, step, max_steps, tol)) break;
         prev = res;
-        subspace_update(d_Vstale, d_wstale, d_U, n, o, w, s);
+        if (const int rc = subspace_update(d_Vstale, d_wstale, d_U, n, o, w, s)) return rc;
     }
     *steps_out = step;
     *res_out = res;
@@ -559,7 +558,7 @@ int subspace_refine_capture(const double *d_Fp, const double *d_Vstale, const do
     if (cudaStreamBeginCaptureToGraph(s_body, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)
         return ERR_CUDA;
     const long long l0 = g_launches;
-    subspace_update(d_Vstale, d_wstale, d_U, n, o, w, s_body);
+    const int rc = subspace_update(d_Vstale, d_wstale, d_U, n, o, w, s_body);
     subspace_residual(d_Fp, d_U, n, o, w, s_body);
     k_refine_decide<<<1, 1, 0, s_body>>>(d_ctl, w.res, h, 0);
     g_launches++;
@@ -567,6 +566,7 @@ int subspace_refine_capture(const double *d_Fp, const double *d_Vstale, const do
     g_launches = l0;
     cudaGraph_t out = nullptr;
     if (cudaStreamEndCapture(s_body, &out) != cudaSuccess) return ERR_CUDA;
+    if (rc) return rc;
     return cudaGetLastError() == cudaSuccess ? OK : ERR_CUDA;
 }
 

@@ -670,8 +670,8 @@ int init_impl(TinySCF_t t, const char *bas_fname, const char *df_bas_fname, cons
         fprintf(stderr, "[tinyscf] shells beyond d (orbital) / f (auxiliary) are not supported\n");
         return ERR_UNSUPPORTED;
     }
-    if (e->ash.nbf > 8192) {   // the J kernels keep one column group of 16 x 512 aux functions per thread block
-        fprintf(stderr, "[tinyscf] %d auxiliary functions: at most 8192 are supported\n", e->ash.nbf);
+    if (e->ash.nbf > MAX_NAUX) {   // the J kernels keep one column group of 16 x 512 aux functions per thread block
+        fprintf(stderr, "[tinyscf] %d auxiliary functions: at most %d are supported\n", e->ash.nbf, MAX_NAUX);
         return ERR_UNSUPPORTED;
     }
     const int nbf = e->sh.nbf, naux = e->ash.nbf;
@@ -2460,7 +2460,7 @@ int batch_refine(TinySCF_batch_t b, const std::vector<int> &todo, std::vector<in
             const double res = *e->h_E;
             cudaStream_t st = f.next();
             if (subspace_continue(res, x.prev, x.step, kRefineSteps, kRefineTol)) {
-                subspace_update(e->V, e->w, e->U, n, o, e->sw, st);
+                RC(subspace_update(e->V, e->w, e->U, n, o, e->sw, st));
                 residual(x.k, st);
                 next.push_back({x.k, res, x.step + 1});
                 continue;

@@ -21,6 +21,7 @@ extern std::atomic<long long> g_eig_launches;
 // ---------------------------------------------------------------- limits
 constexpr int MAX_L_ORB = 2;           // orbital shells up to d
 constexpr int MAX_L_AUX = 3;           // auxiliary shells up to f
+constexpr int MAX_NAUX = 8192;         // auxiliary functions (the J kernels: one group of 16 x 512 columns per block)
 constexpr int MAXDIIS  = 10;          // TinySCF.h:8
 constexpr int BOYS_MMAX = 8;           // highest F_m needed: (dd|dd) Schwarz quartets
 constexpr int BOYS_TAYLOR = 7;         // Taylor terms of the tabulated Boys function
@@ -305,8 +306,8 @@ struct SubspaceWork {
 int subspace_refine(const double *d_Fp, const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o,
                     SubspaceWork &w, double tol, int max_steps, int *steps_out, double *res_out, cudaStream_t s);
 void subspace_residual(const double *d_Fp, const double *d_U, int n, int o, SubspaceWork &w, cudaStream_t s);   // into w.res
-void subspace_update(const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o, SubspaceWork &w,
-                     cudaStream_t s);
+int subspace_update(const double *d_Vstale, const double *d_wstale, double *d_U, int n, int o, SubspaceWork &w,
+                    cudaStream_t s);
 bool subspace_continue(double res, double prev, int step, int max_steps, double tol);
 // Refinement inside a stream capture: the steps run in a WHILE conditional
 // node whose condition a device kernel sets from the residual. d_ctl->tol and
