@@ -321,8 +321,8 @@ __device__ __forceinline__ double u128_to_double(u128 x)
 // columns of a row: lane = 8 g + q reads the residues of columns 4 q .. 4 q + 3
 // (one 32-bit word; sums over at most 256 ranges of 255 stay in 16 bits) for
 // the moduli g, g + 4, ..., whose terms are added unreduced (16 M < 2^122)
-// and meet by shuffles. nbf = 510 in 24 ranges: 269 us, now 91 us; 325 in 37: 131 us,
-// now 26 us (one group per range, 1010 in 5: 187 us, now 232 us).
+// and meet by shuffles. nbf = 510 in 24 ranges: 269 us with k_oz_crt_ranges below, now
+// 91 us; 325 in 37: 131 us, now 26 us.
 constexpr int OZ_CRT_COLS = 4, OZ_CRT_WCOLS = 32;
 __global__ void __launch_bounds__(128) k_oz_crt(const uint8_t *__restrict__ res, int nsplit, int group, int nmod,
                                                 int rows_pad, int nbf, const int *__restrict__ e, int beta, double *K)
@@ -381,6 +381,38 @@ __global__ void __launch_bounds__(128) k_oz_crt(const uint8_t *__restrict__ res,
     }
     const int j = j0 + mg;
     if (j < i || j >= nbf) return;
+    const double v = pos >= neg ? u128_to_double(pos - neg) : -u128_to_double(neg - pos);
+    const double kv = ldexp(v, e[i] + e[j] - 2 * beta);
+    K[(size_t) i * nbf + j] = kv;
+    K[(size_t) j * nbf + i] = kv;
+}
+
+// The same, an element a thread, where every range is a group of its own: there
+// is nothing to add up before the CRT then, and its independent loads are worth
+// more than the shared words and shuffles (us here / above: nbf = 1010 in 7 ranges
+// 186 / 232, 935 179 / 225, 885 163 / 188, 800 137 / 168; with two ranges a group
+// 860 155 / 146, 785 138 / 138).
+__global__ void k_oz_crt_ranges(const uint8_t *__restrict__ res, int nsplit, int nmod, int rows_pad, int nbf,
+                                const int *__restrict__ e, int beta, double *K)
+{
+    const long long idx = (long long) blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long) nbf * nbf) return;
+    const int i = (int) (idx / nbf), j = (int) (idx % nbf);
+    if (i > j) return;
+    const u128 M = ((u128) c_M[1] << 64) | c_M[0];
+    const u128 half = M >> 1;
+    u128 pos = 0, neg = 0;   // total = pos - neg
+    for (int r = 0; r < nsplit; r++) {
+        u128 acc = 0;
+        for (int k = 0; k < nmod; k++) {
+            const uint32_t v = res[(((size_t) r * nmod + k) * rows_pad + i) * rows_pad + j];
+            const uint32_t s = (v * (uint32_t) c_y[k]) % (uint32_t) c_mi[k];
+            acc += (u128) s * (((u128) c_Mk[k][1] << 64) | c_Mk[k][0]);
+            if (acc >= M) acc -= M;
+        }
+        if (acc > half) neg += M - acc;
+        else pos += acc;
+    }
     const double v = pos >= neg ? u128_to_double(pos - neg) : -u128_to_double(neg - pos);
     const double kv = ldexp(v, e[i] + e[j] - 2 * beta);
     K[(size_t) i * nbf + j] = kv;
@@ -544,10 +576,16 @@ int oz_syrk(OzSyrk *o, const double *d_T, double *d_K, cudaStream_t s, const uns
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (cudaLaunchKernelEx(&cfg, k_oz_gemm, o->mR, a) != cudaSuccess) return ERR_CUDA;
-    const long long nw = (long long) o->nbf * ((o->nbf + OZ_CRT_WCOLS - 1) / OZ_CRT_WCOLS);
     const int group = std::max(1, std::min(256, OZ_MAX_CHUNKS / o->cps));
-    k_oz_crt<<<(unsigned) ((nw + 3) / 4), 128, 0, s>>>(o->res, o->ksplit, group, o->nmod, o->rows_pad, o->nbf, o->e,
+    if (group == 1) {
+        const long long nn = (long long) o->nbf * o->nbf;
+        k_oz_crt_ranges<<<(unsigned) ((nn + 255) / 256), 256, 0, s>>>(o->res, o->ksplit, o->nmod, o->rows_pad, o->nbf,
+                                                                     o->e, o->beta, d_K);
+    } else {
+        const long long nw = (long long) o->nbf * ((o->nbf + OZ_CRT_WCOLS - 1) / OZ_CRT_WCOLS);
+        k_oz_crt<<<(unsigned) ((nw + 3) / 4), 128, 0, s>>>(o->res, o->ksplit, group, o->nmod, o->rows_pad, o->nbf, o->e,
                                                           o->beta, d_K);
+    }
     g_launches += 4;
     return cuda_launch_rc("Ozaki rank-k product");
 }
