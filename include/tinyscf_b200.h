@@ -292,6 +292,14 @@ TINYSCF_API int TinySCF_wait_probe(TinySCF_t t, long long wait_cycles);
  * device; synchronous. TINYSCF_ERR_CUDA if a grid barrier of the
  * tridiagonalisation gave up waiting. */
 TINYSCF_API int TinySCF_eigh(int device, int n, const double *A, double *w, double *V);
+/* The same with the stopping rule of the roots in divide and conquer:
+ * TINYSCF_EIG_NOISE (TinySCF_eigh; the plain form's density) stops where the
+ * secular equation's value is rounding, TINYSCF_EIG_BRACKET (X, (P|Q)^-1/2 and
+ * the accelerated form's eigenbases, whose users amplify the last bits) where
+ * the root's bracket closes. */
+#define TINYSCF_EIG_BRACKET 0
+#define TINYSCF_EIG_NOISE   1
+TINYSCF_API int TinySCF_eigh_stop(int device, int n, const double *A, double *w, double *V, int stop);
 /* K = T T^T (T: n x q, row-major; K: n x n, both triangles) on host buffers,
  * by the integer-tensor-core product the engine's FP64 exchange uses when
  * TINYSCF_OZAKI selects it (the rank-k step of build_Fock.c:317-341): each row

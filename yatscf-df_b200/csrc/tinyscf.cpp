@@ -2794,6 +2794,12 @@ int TinySCF_wait_probe(TinySCF_t t, long long wait_cycles)
 
 int TinySCF_eigh(int device, int n, const double *A, double *w, double *V)
 {
+    return TinySCF_eigh_stop(device, n, A, w, V, TINYSCF_EIG_NOISE);
+}
+
+int TinySCF_eigh_stop(int device, int n, const double *A, double *w, double *V, int stop)
+{
+    if (stop != TINYSCF_EIG_NOISE && stop != TINYSCF_EIG_BRACKET) return TINYSCF_ERR_INPUT;
     if (n < 1 || n > EIG_MAX_N || !A || !w || !V) return TINYSCF_ERR_INPUT;
     if (cudaSetDevice(device) != cudaSuccess) return TINYSCF_ERR_CUDA;
     cudaStream_t s = nullptr;
@@ -2809,7 +2815,7 @@ int TinySCF_eigh(int device, int n, const double *A, double *w, double *V)
         rc = TINYSCF_ERR_CUDA;
     } else {
         unsigned mark = waits_mark();
-        rc = eig_run(eg, dA, dw, dV, s, true);
+        rc = eig_run(eg, dA, dw, dV, s, stop == TINYSCF_EIG_NOISE);
         if (rc == OK && (cudaMemcpyAsync(w, dw, sizeof(double) * n, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaMemcpyAsync(V, dV, sizeof(double) * nn, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaStreamSynchronize(s) != cudaSuccess))

@@ -128,6 +128,7 @@ def load_library(path=LIBPATH):
                                  ctypes.c_longlong], ctypes.c_longlong),
         "quickSort_eigval": ([dp, ctypes.POINTER(ctypes.c_int), ip, ip], None),
         "TinySCF_eigh": ([ip, ip, dp, dp, dp], ip),
+        "TinySCF_eigh_stop": ([ip, ip, dp, dp, dp, ip], ip),
         "TinySCF_syrk_int8": ([ip, ip, ctypes.c_longlong, dp, dp], ip),
         "TinySCF_trim_memory": ([ip], ip),
         "TinySCF_kmix_wait_probe": ([T, ctypes.c_longlong, ctypes.POINTER(ctypes.c_int)], ip),
@@ -472,15 +473,19 @@ def set_autotune(on):
     load_library().TinySCF_set_autotune(int(bool(on)))
 
 
-def eigh(A, device=0):
+EIG_BRACKET, EIG_NOISE = 0, 1
+
+
+def eigh(A, device=0, stop=EIG_NOISE):
     """(w, V) of a symmetric matrix from the engine's device eigensolver:
-    eigenvalues ascending, V[k] the k-th eigenvector."""
+    eigenvalues ascending, V[k] the k-th eigenvector; stop: which rule ends the
+    roots of divide and conquer."""
     lib = load_library()
     A = np.ascontiguousarray(A, dtype=np.float64)
     n = A.shape[0]
     w = np.zeros(n)
     V = np.zeros((n, n))
-    rc = lib.TinySCF_eigh(int(device), n, _dptr(A), _dptr(w), _dptr(V))
+    rc = lib.TinySCF_eigh_stop(int(device), n, _dptr(A), _dptr(w), _dptr(V), int(stop))
     if rc:
         raise TinySCFError("eigh: " + STATUS.get(rc, str(rc)))
     return w, V
