@@ -1152,7 +1152,8 @@ __device__ __forceinline__ void secular_parts(const double *sd, const double *sz
 // bracket's end, so most roots go through tens of bisections of a wide bracket
 // before it closes (50 us per level however few roots). at_noise stops where
 // |f| is within the rounding of its own terms instead, which determines the root
-// as far as f can (the criterion of LAPACK's dlaed4): 13 us. The bracketed
+// as far as f can (the criterion of LAPACK's dlaed4, whose eps is the unit
+// roundoff DBL_EPSILON / 2): 13 us. The bracketed
 // stop stays for the eigenbases of the accelerated form and of X and (P|Q)^-1/2,
 // whose users amplify the last bits (1e-16 in X moves its density by 1e-9).
 // One warp; the root of position j as org, tau (tau relative to sd[org]).
@@ -1194,7 +1195,7 @@ __device__ __forceinline__ void secular_root(const double *sd, const double *sz,
             secular_parts(sd, sz, k, j, rho, dorg, tau, lane, p1, dp1, p2, dp2);
             const double f = 1.0 + p1 + p2;
             if (f == 0.0) break;
-            if (at_noise && fabs(f) <= DBL_EPSILON * (8.0 * (1.0 + fabs(p1) + fabs(p2)) + fabs(tau) * (dp1 + dp2))) break;
+            if (at_noise && fabs(f) <= 0.5 * DBL_EPSILON * (8.0 * (1.0 + fabs(p1) + fabs(p2)) + fabs(tau) * (dp1 + dp2))) break;
             if (f < 0.0) a = tau; else b = tau;
             if (!(b - a > 4.0 * DBL_EPSILON * fmax(fabs(a), fabs(b)))) break;
             // two-pole model: C + s1 / (del1 - x) + s2 / (del2 - x) = 0
