@@ -225,8 +225,13 @@ TINYSCF_API int TinySCF_device_memory(int device, long long *free_bytes, long lo
  * memory pool, which keeps memory reserved after an engine is freed so that
  * the next engine reuses it without new mappings (TINYSCF_MEMPOOL=0 in the
  * environment uses cudaMalloc / cudaFree instead). This returns the pool's
- * unused memory to the device. */
+ * unused memory to the device. It also unlocks the page-locked host memory that
+ * freed engines left for the next ones (at most 256 MB a process, live and idle
+ * together; what does not fit is pageable). */
 TINYSCF_API int TinySCF_trim_memory(int device);
+/* Page-locked host memory of the process's engines in bytes: held by engines,
+ * and idle (which TinySCF_trim_memory gives back). Either pointer may be NULL. */
+TINYSCF_API int TinySCF_pinned_memory(long long *live_bytes, long long *idle_bytes);
 /* The tuner's table as text ("key -> choice (ms) [candidate: ms]..."); writes
  * at most len bytes into buf and returns the full length. */
 TINYSCF_API int TinySCF_autotune_report(char *buf, int len);

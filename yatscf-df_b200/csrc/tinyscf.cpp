@@ -518,17 +518,17 @@ std::mutex &amaps_mu()
 
 // Page-locked host blocks. A process keeps at most PIN_MAX bytes of them,
 // live and idle together; what engines give back waits here for the next engine
-// of the same sizes, since locking and unlocking pages (and freeing any driver
+// of the same sizes (or for TinySCF_trim_memory), since locking and unlocking pages (and freeing any driver
 // allocation) goes through the kernel driver: 8 MB take 2 to 4 ms, and on a
 // machine whose driver is busy with other processes one cudaFreeHost was seen to
 // take 0.2 to 0.8 s of a job of 0.5 s. Idle blocks of other sizes make room.
 class PinPool {
     static constexpr size_t PIN_MAX = (size_t) 256 << 20, PIN_ROUND = (size_t) 64 << 10;
-    static constexpr int SLOT = 256, SLOTS = 64;   // small blocks: slots of a slab that stays
+    static constexpr int SLOT = 256, SLOTS = 64;   // small blocks: slots of slabs
     std::mutex mu_;
     std::map<void *, size_t> live_;
     std::multimap<size_t, void *> idle_;
-    std::vector<void *> slots_;
+    std::vector<void *> slots_, slabs_;   // free slots; their slabs
     size_t total_ = 0;
 
 public:
@@ -581,6 +581,7 @@ public:
                 cudaGetLastError();
                 return nullptr;
             }
+            slabs_.push_back(b);
             for (int k = 0; k < SLOTS; k++) slots_.push_back(b + k * SLOT);
         }
         void *p = slots_.back();
@@ -592,6 +593,30 @@ public:
         if (!p) return;
         std::lock_guard<std::mutex> lk(mu_);
         slots_.push_back(p);
+    }
+    // Unlocks what no engine holds (the slabs once all their slots are back).
+    void trim()
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        for (auto &b : idle_) {
+            cudaFreeHost(b.second);
+            total_ -= b.first;
+        }
+        idle_.clear();
+        if (slots_.size() == slabs_.size() * SLOTS) {
+            for (void *b : slabs_) cudaFreeHost(b);
+            slots_.clear();
+            slabs_.clear();
+        }
+    }
+    void sizes(long long *live, long long *idle)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        size_t n = 0;
+        for (auto &b : idle_) n += b.first;
+        const size_t used = slabs_.size() * SLOTS - slots_.size();
+        *live = (long long) (total_ - n + used * SLOT);
+        *idle = (long long) (n + slots_.size() * SLOT);
     }
     static_assert(sizeof(RefineCtl) <= SLOT, "a slot holds the refinement's control block");
 };
@@ -2839,8 +2864,18 @@ int TinySCF_trim_memory(int device)
     }
     if (cudaSetDevice(device) != cudaSuccess) return TINYSCF_ERR_CUDA;
     const int rc = dev_trim(device);
+    PinPool::get().trim();
     cudaSetDevice(cur);
     return rc == OK ? TINYSCF_OK : TINYSCF_ERR_CUDA;
+}
+
+int TinySCF_pinned_memory(long long *live_bytes, long long *idle_bytes)
+{
+    long long live = 0, idle = 0;
+    PinPool::get().sizes(&live, &idle);
+    if (live_bytes) *live_bytes = live;
+    if (idle_bytes) *idle_bytes = idle;
+    return TINYSCF_OK;
 }
 
 int TinySCF_syrk_int8(int device, int n, long long q, const double *T, double *K)

@@ -131,6 +131,7 @@ def load_library(path=LIBPATH):
         "TinySCF_eigh_stop": ([ip, ip, dp, dp, dp, ip], ip),
         "TinySCF_syrk_int8": ([ip, ip, ctypes.c_longlong, dp, dp], ip),
         "TinySCF_trim_memory": ([ip], ip),
+        "TinySCF_pinned_memory": ([ctypes.POINTER(ctypes.c_longlong)] * 2, ip),
         "TinySCF_kmix_wait_probe": ([T, ctypes.c_longlong, ctypes.POINTER(ctypes.c_int)], ip),
         "TinySCF_wait_probe": ([T, ctypes.c_longlong], ip),
         "TinySCF_set_aux_slice": ([T, ip, ip], ip),
@@ -491,8 +492,15 @@ def eigh(A, device=0, stop=EIG_NOISE):
     return w, V
 
 
+def pinned_memory():
+    """(held, idle) bytes of the engines' page-locked host memory."""
+    live, idle = ctypes.c_longlong(0), ctypes.c_longlong(0)
+    load_library().TinySCF_pinned_memory(ctypes.byref(live), ctypes.byref(idle))
+    return live.value, idle.value
+
+
 def trim_memory(device=0):
-    """Return the memory that freed engines left in the device's pool."""
+    """Return the memory that freed engines left in the device's pool, and their page-locked host memory."""
     rc = load_library().TinySCF_trim_memory(int(device))
     if rc:
         raise TinySCFError("trim_memory: " + STATUS.get(rc, str(rc)))
