@@ -305,6 +305,10 @@ TINYSCF_API int TinySCF_eigh(int device, int n, const double *A, double *w, doub
 #define TINYSCF_EIG_BRACKET 0
 #define TINYSCF_EIG_NOISE   1
 TINYSCF_API int TinySCF_eigh_stop(int device, int n, const double *A, double *w, double *V, int stop);
+/* FP64 products of the process so far that ran on the TMA-fed 168 x 96 tiles
+ * (large row-major products in whole 16-byte units, the DF tensor's among them;
+ * the others take the tiles that need no alignment). */
+TINYSCF_API long long TinySCF_gemm_bulk_count(void);
 /* K = T T^T (T: n x q, row-major; K: n x n, both triangles) on host buffers,
  * by the integer-tensor-core product the engine's FP64 exchange uses when
  * TINYSCF_OZAKI selects it (the rank-k step of build_Fock.c:317-341): each row

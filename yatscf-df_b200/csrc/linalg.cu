@@ -21,7 +21,7 @@
 
 namespace tscf {
 
-std::atomic<long long> g_launches{0};
+std::atomic<long long> g_launches{0}, g_bulk_gemms{0};
 
 // the pools of fork.h outlive static destruction
 std::mutex &Fork::lock()
@@ -249,6 +249,7 @@ static bool dgemm_bulk(int m, int n, int k, double alpha, const double *A, int l
     k_dgemm_bulk<<<std::min(ntiles, num_sms()), BG_THREADS, BG_SMEM, s>>>(mA, mB, m, n, k, alpha, C, ldc, ntn, ntiles,
                                                                                wait_word());
     g_launches++;
+    g_bulk_gemms++;
     return true;
 }
 

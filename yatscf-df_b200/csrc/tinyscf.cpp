@@ -2878,6 +2878,8 @@ int TinySCF_pinned_memory(long long *live_bytes, long long *idle_bytes)
     return TINYSCF_OK;
 }
 
+long long TinySCF_gemm_bulk_count(void) { return g_bulk_gemms; }
+
 int TinySCF_syrk_int8(int device, int n, long long q, const double *T, double *K)
 {
     if (n < 1 || q < 1 || !T || !K) return TINYSCF_ERR_INPUT;

@@ -134,6 +134,7 @@ int      waits_check(unsigned &mark, const char *what);
 int      waits_take();   // the word's code (0: none), taken as reported
 // Stores the code of a wait that runs out after `cycles` (a barrier that nothing completes), to test the reports.
 int      wait_probe(long long cycles, cudaStream_t s);
+extern std::atomic<long long> g_bulk_gemms;   // products that ran on the producer-warp tiles (linalg.cu)
 // The same product with the tile picked from the call shape (no tuning run).
 void dgemm_untuned(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int lda,
                    const double *B, int ldb, double beta, double *C, int ldc, cudaStream_t s);

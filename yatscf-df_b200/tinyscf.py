@@ -131,6 +131,7 @@ def load_library(path=LIBPATH):
         "TinySCF_eigh_stop": ([ip, ip, dp, dp, dp, ip], ip),
         "TinySCF_syrk_int8": ([ip, ip, ctypes.c_longlong, dp, dp], ip),
         "TinySCF_trim_memory": ([ip], ip),
+        "TinySCF_gemm_bulk_count": ([], ctypes.c_longlong),
         "TinySCF_pinned_memory": ([ctypes.POINTER(ctypes.c_longlong)] * 2, ip),
         "TinySCF_kmix_wait_probe": ([T, ctypes.c_longlong, ctypes.POINTER(ctypes.c_int)], ip),
         "TinySCF_wait_probe": ([T, ctypes.c_longlong], ip),
@@ -504,6 +505,11 @@ def trim_memory(device=0):
     rc = load_library().TinySCF_trim_memory(int(device))
     if rc:
         raise TinySCFError("trim_memory: " + STATUS.get(rc, str(rc)))
+
+
+def gemm_bulk_count():
+    """FP64 products of this process that ran on the TMA-fed tiles."""
+    return load_library().TinySCF_gemm_bulk_count()
 
 
 def syrk_int8(T, device=0):
