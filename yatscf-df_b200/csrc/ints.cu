@@ -4,16 +4,19 @@
 // (libCMS/CMS_Simint.c:363 4-centre, :411 overlap, :441/:444 kinetic+nuclear,
 // :527 batched 3-centre, :595 2-centre).
 //
-// Work is bucketed by angular-momentum class so every warp runs one class:
-// one launch per (la,lb[,lc]) class, a group of lanes per shell pair (1e,
-// Schwarz) or (shell pair, aux shell) triplet (3-centre), which share its
-// primitive pairs, and one thread per aux pair (2-centre). The recursions are
-// unrolled with constant indices (ints_unrolled.cuh).
+// Work is bucketed by angular-momentum class so every warp runs one class: one
+// launch per (la,lb[,lc]) class. The Schwarz kernel gives a shell pair a group of
+// lanes that share its primitive pairs; it and the DF screening values run on
+// recursions unrolled with constant indices (ints_unrolled.cuh). The one-electron,
+// 2-centre and 3-centre kernels take one thread per shell pair, aux pair or (shell
+// pair, aux shell) triplet and run the recursions below with run-time loops: their
+// values enter S^-1/2 and (P|Q)^-1/2, which amplify the last bits, and the unrolled
+// forms round differently.
 //
 // Conventions: Cartesian components in lexicographic order (xx,xy,xz,yy,yz,zz);
-// contracted shells normalised so the x^l component has unit norm; a second
-// exponent of 0 turns 4-centre into 3-/2-centre integrals, as the unit shell
-// of libCMS/CMS_Simint.c:131-141 does.
+// contracted shells normalised so the x^l component has unit norm; the "unit
+// shell" (exponent 0, coefficient 1) turns 4-centre into 3-/2-centre integrals, as
+// in libCMS/CMS_Simint.c:131-141 (a second exponent of 0 in the DF screening values).
 #include <cmath>
 #include <cstdio>
 #include <vector>
