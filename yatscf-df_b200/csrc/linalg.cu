@@ -40,7 +40,8 @@ std::vector<Fork::Set *> &Fork::pool(int dev)
 // matrices) and 128x64 (more reuse for large ones) (dgemm_tile), and 128x128
 // and 64x64 on the FP64 tensor cores (dgemm_tile_dmma, dgemm_tile_dmma64). The
 // autotuner picks one per call shape the first time the shape is met outside
-// a stream capture.
+// a stream capture; they sum over k in the same order. A sixth, K split over
+// warps (k_dgemm_dmma32ks), rounds differently and goes by a rule (ksplit_order).
 template <bool TA, bool TB, int BM, int BN>
 __global__ void __launch_bounds__(256) k_dgemm(int m, int n, int k, double alpha, const double *__restrict__ A, int lda,
                                                const double *__restrict__ B, int ldb, double beta, double *C, int ldc)
